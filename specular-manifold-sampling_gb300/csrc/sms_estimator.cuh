@@ -270,6 +270,8 @@ SMS_D bool ss_newton(const DevScene &sc, const SolverCfg &cfg, f3 x, f3 lp, Vtx 
                                   : step_anglediff(x, v, lp, c0, c1, dx0, dx1, no);
         if (!sok) break;
         if (sqrtf(c0 * c0 + c1 * c1) < cfg.solver_threshold) { conv = true; break; }
+        // the last iteration's ray would lead to a vertex no step is taken from
+        if (it + 1 >= cfg.max_iterations) { it++; break; }
         f3 pp = v.p - (v.dp_du * dx0 + v.dp_dv * dx1) * (cfg.step_scale * beta);
         f3 dd = normalize(pp - x);
         trace<kTree>(sc, x, dd, kRayEps, INFINITY, false, h, err);

@@ -358,6 +358,8 @@ SMS_D bool chain_newton(const DevScene &sc, const SolverCfg &cfg, f3 x0, f3 lp, 
         if (need) ok = chain_step<K, kRough>(cfg, x0, lp, c, conv, du, dv, offs);
         if (!ok) break;
         if (conv) break;
+        // the last iteration's chain would be one no step is taken from
+        if (it + 1 >= cfg.max_iterations) { it++; break; }
         f3 p0 = c.v[0].p - (c.v[0].dp_du * du + c.v[0].dp_dv * dv) * (cfg.step_scale * beta);
         Chain<K> prop;
         if (trace_chain<K, kNM, kRough>(sc, x0, p0, tmpl, false, prop, nullptr, err, st, false, co)) {
