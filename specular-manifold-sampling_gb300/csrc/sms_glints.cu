@@ -395,36 +395,38 @@ __global__ void __launch_bounds__(128, 8) glint_biased_kernel(DevScene sc, Solve
                 st.newton += (unsigned)it;
                 if (ok) st.succ++; else st.fail++;
             }
+            // first occurrences in walk order: one pass per converged walk
             bool keep = false;
-            for (int k = 0; k < G; ++k) {
-                const int src = gbase + k;
-                bool ck = __shfl_sync(kFullG, ok, src);
+            unsigned pend = __ballot_sync(kFullG, ok) & gmask;
+            while (__any_sync(kFullG, pend != 0u)) {
+                const int src = pend ? __ffs(pend) - 1 : (int)lane;
                 f2 uk = {__shfl_sync(kFullG, uv.x, src), __shfl_sync(kFullG, uv.y, src)};
                 bool dup = false;
-                if (ck)
+                if (pend)
                     for (int j = gl; j < nrec; j += G) {
                         float dx = uk.x - rec[gib][j].x, dy = uk.y - rec[gib][j].y;
                         if (sqrtf(dx * dx + dy * dy) < cfg.uniqueness_threshold) dup = true;
                     }
                 unsigned anydup = __ballot_sync(kFullG, dup) & gmask;
                 __syncwarp();
-                if (ck && !anydup) {
+                if (pend && !anydup) {
                     if (nrec < kMaxSolutions) {
                         if (gl == 0) rec[gib][nrec] = uk;
                         nrec++;
-                        if (gl == k) keep = true;
+                        if ((int)lane == src) keep = true;
                     } else {
                         err |= kErrSolutionOverflow;
                     }
                 }
+                pend &= pend - 1u;
                 __syncwarp();
             }
             float c = keep ? glint_contribution(sc, Q, L, uv, err, st) : 0.f;
-            for (int k = 0; k < G; ++k) {
-                const int src = gbase + k;
-                bool kk = __shfl_sync(kFullG, keep, src);
-                float ck = __shfl_sync(kFullG, c, src);
-                if (kk) acc += ck;
+            pend = __ballot_sync(kFullG, keep) & gmask;
+            while (__any_sync(kFullG, pend != 0u)) {
+                const float ck = __shfl_sync(kFullG, c, pend ? __ffs(pend) - 1 : (int)lane);
+                if (pend) acc += ck;
+                pend &= pend - 1u;
             }
         }
         if (live && gl == 0) {

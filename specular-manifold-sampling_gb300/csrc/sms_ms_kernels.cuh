@@ -730,38 +730,40 @@ __global__ void __launch_bounds__(128, SMS_MS_BIASED_MIN_BLOCKS) ms_biased_kerne
                 f3 dir = ok ? normalize(c.v[0].p - Q.x) : splat(0.f);
                 // walk-ordered deduplication (no visibility test first, :162-184)
                 bool keep = false;
-                for (int k = 0; k < G; ++k) {
-                    const int src = gbase + k;
-                    bool ck = __shfl_sync(kFull, ok, src);
+                unsigned pend = __ballot_sync(kFull, ok) & gmask;
+                while (__any_sync(kFull, pend != 0u)) {
+                    const int src = pend ? __ffs(pend) - 1 : (int)lane;
                     f3 dk = mk(__shfl_sync(kFull, dir.x, src), __shfl_sync(kFull, dir.y, src),
                                __shfl_sync(kFull, dir.z, src));
                     bool dup = false;
-                    if (ck)
+                    if (pend)
                         for (int j = gl; j < nrec; j += G)
                             if (fabsf(dot(dk, rec[gib][j]) - 1.f) < cfg.uniqueness_threshold) dup = true;
                     unsigned anydup = __ballot_sync(kFull, dup) & gmask;
                     __syncwarp();
-                    if (ck && !anydup) {
+                    if (pend && !anydup) {
                         if (nrec < kMaxSolutions) {
                             if (gl == 0) rec[gib][nrec] = dk;
                             nrec++;
-                            if (gl == k) keep = true;
+                            if ((int)lane == src) keep = true;
                         } else {
                             err |= kErrSolutionOverflow;
                         }
                     }
+                    pend &= pend - 1u;
                     __syncwarp();
                 }
                 f3 contrib = splat(0.f);
                 if (keep)
                     contrib = receiver_eval(sc, Q, dir, err) * chain_contribution<K, kNM, kRough>(sc, Q.x, L, c, err, st);
                 // sum in walk order
-                for (int k = 0; k < G; ++k) {
-                    const int src = gbase + k;
-                    bool kk = __shfl_sync(kFull, keep, src);
+                pend = __ballot_sync(kFull, keep) & gmask;
+                while (__any_sync(kFull, pend != 0u)) {
+                    const int src = pend ? __ffs(pend) - 1 : (int)lane;
                     f3 vk = mk(__shfl_sync(kFull, contrib.x, src), __shfl_sync(kFull, contrib.y, src),
                                __shfl_sync(kFull, contrib.z, src));
-                    if (kk) cur = cur + vk;
+                    if (pend) cur = cur + vk;
+                    pend &= pend - 1u;
                 }
             }
             // result += value / m_offset_normals_pdf (:198)

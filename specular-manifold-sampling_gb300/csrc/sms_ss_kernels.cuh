@@ -111,21 +111,21 @@ __global__ void __launch_bounds__(128, 4) ss_biased_kernel(DevScene sc, SolverCf
                         st.fail++;
                     }
                 }
-                // walk-ordered deduplication within the group
-                for (int k = 0; k < G; ++k) {
-                    const int src = gbase + k;
-                    bool ck = __shfl_sync(full, cand, src);
+                // walk-ordered deduplication within the group, one pass per candidate
+                unsigned pend = __ballot_sync(full, cand) & gmask;
+                while (__any_sync(full, pend != 0u)) {
+                    const int src = pend ? __ffs(pend) - 1 : (int)lane;
                     f3 dk = mk(__shfl_sync(full, dir.x, src), __shfl_sync(full, dir.y, src),
                                __shfl_sync(full, dir.z, src));
                     f3 vk = mk(__shfl_sync(full, contrib.x, src), __shfl_sync(full, contrib.y, src),
                                __shfl_sync(full, contrib.z, src));
                     bool dup = false;
-                    if (ck)
+                    if (pend)
                         for (int j = gl; j < nrec; j += G)
                             if (fabsf(dot(dk, rec[gib][j]) - 1.f) < cfg.uniqueness_threshold) dup = true;
                     unsigned anydup = __ballot_sync(full, dup) & gmask;
                     __syncwarp();
-                    if (ck && !anydup) {
+                    if (pend && !anydup) {
                         if (nrec < kMaxSolutions) {
                             if (gl == 0) rec[gib][nrec] = dk;
                             nrec++;
@@ -134,6 +134,7 @@ __global__ void __launch_bounds__(128, 4) ss_biased_kernel(DevScene sc, SolverCf
                             err |= kErrSolutionOverflow;
                         }
                     }
+                    pend &= pend - 1u;
                     __syncwarp();
                 }
             }
