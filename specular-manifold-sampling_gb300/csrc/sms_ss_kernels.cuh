@@ -28,6 +28,11 @@ namespace sms {
 #ifndef SMS_SS_WALK_MIN_BLOCKS
 #define SMS_SS_WALK_MIN_BLOCKS 9
 #endif
+// Normal-mapped casters: the map's frame and the two-stage solver add
+// arithmetic, not traversal, so what counts is that the step stays in
+// registers.  4 blocks (128 registers); normal-mapped pane with the
+// two-stage solver at 4 and 9 blocks: 0.69 and 0.83 ms (15,203 points, conductor).
+constexpr int ss_walk_blocks(int var) { return (var & 4) ? 4 : SMS_SS_WALK_MIN_BLOCKS; }
 
 // ------------------------------------------------------ biased estimator
 // Group of G lanes per query; walk m of caster c sits at stream position
@@ -158,7 +163,7 @@ __global__ void __launch_bounds__(128, 4) ss_biased_kernel(DevScene sc, SolverCf
 // mlp::proposal_seed, mixture from ss_proposal_kernel) instead of two-draw
 // uniform seeding.
 template <bool kLearned, int kVar>
-__global__ void __launch_bounds__(128, SMS_SS_WALK_MIN_BLOCKS) ss_first_kernel(DevScene sc, SolverCfg cfg, int c, const float *__restrict__ qs,
+__global__ void __launch_bounds__(128, ss_walk_blocks(kVar)) ss_first_kernel(DevScene sc, SolverCfg cfg, int c, const float *__restrict__ qs,
                                                        uint32_t n, uint64_t seed, uint64_t stream_off,
                                                        float *__restrict__ value, int *__restrict__ count,
                                                        int *__restrict__ walks, SsScratch scr, DevCounters *ctr,
@@ -271,7 +276,7 @@ __global__ void __launch_bounds__(128, SMS_SS_WALK_MIN_BLOCKS) ss_first_kernel(D
 // All lanes run one warp-uniform loop: groups whose query finished fetch the
 // next one at the top, so every ballot and shuffle has the whole warp.
 template <bool kLearned, int G, int kVar, bool kTree = false>
-__global__ void __launch_bounds__(128, SMS_SS_WALK_MIN_BLOCKS) ss_trials_kernel(DevScene sc, SolverCfg cfg, int c, const float *__restrict__ qs,
+__global__ void __launch_bounds__(128, ss_walk_blocks(kVar)) ss_trials_kernel(DevScene sc, SolverCfg cfg, int c, const float *__restrict__ qs,
                                                         uint32_t n, uint64_t seed, uint64_t stream_off,
                                                         float *__restrict__ value, int *__restrict__ count,
                                                         int *__restrict__ walks, SsScratch scr, DevCounters *ctr,
