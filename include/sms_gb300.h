@@ -216,11 +216,10 @@ void      *sms_ctx_stream(sms_ctx *ctx);
 /* Launch shape of the persistent kernels: blocks per SM and threads per block
  * (0 = library default).  Set by the autotuner. */
 sms_status sms_ctx_set_launch(sms_ctx *ctx, int32_t blocks_per_sm, int32_t threads_per_block);
-/* Lanes per query of the unbiased estimator's Bernoulli-trial kernel: 8, 16
- * or 32 trials of one query run side by side (the first success is found by
- * ballot, so results do not depend on it); 0 picks 32 for uniform seeding and
- * 8 with a learned proposal.  No counterpart in the reference (a tuning knob
- * of the batched solver). */
+/* Lanes of a warp of the single-scatter Bernoulli-trial kernel that take
+ * trials, one each: 8, 16 or 32 (0 = 32).  Fewer lanes wait less for each
+ * other and use less of the machine; results do not depend on it.  No
+ * counterpart in the reference (a tuning knob of the batched solver). */
 sms_status sms_ctx_set_trial_group(sms_ctx *ctx, int32_t group);
 /* Top node records of the scene's tree (stored breadth first) that the
  * Bernoulli-trial kernel copies into each block's shared memory before it
@@ -228,9 +227,10 @@ sms_status sms_ctx_set_trial_group(sms_ctx *ctx, int32_t group);
  * L1 for the top levels; results do not depend on it.  No counterpart in the
  * reference (a staging knob of the batched solver, set by the autotuner). */
 sms_status sms_ctx_set_treelet(sms_ctx *ctx, int32_t nodes);
-/* Queries a lane group of the Bernoulli-trial kernel claims from the work queue
- * per atomic, 1..64 (default 1).  Results do not depend on it.  No counterpart
- * in the reference (a tuning knob of the batched solver, set by the autotuner). */
+/* Rounds of trials a warp of the Bernoulli-trial kernel claims from the stream
+ * of trials per atomic, at least; 1..64 (default 1).  Results do not depend on
+ * it.  No counterpart in the reference (a tuning knob of the batched solver,
+ * set by the autotuner). */
 sms_status sms_ctx_set_queue_chunk(sms_ctx *ctx, int32_t chunk);
 
 /* ---------------------------------------------------------------- queries */
@@ -276,14 +276,16 @@ typedef struct sms_stats {
     uint64_t bernoulli_trial_iterations;
     uint64_t bernoulli_trial_iterations_max;
     uint64_t walks;
-    uint64_t newton_iterations;
+    uint64_t newton_iterations;   /* of the walks counted in walks, plus those
+                                     of speculative trials that ended before
+                                     the success that made them speculative */
     uint64_t connections;
     uint64_t rays;          /* rays cast by the connection kernel        */
     uint64_t bvh_nodes;     /* BVH nodes fetched (64 bytes each)         */
     uint64_t tri_tests;     /* triangles fetched (48 bytes each)         */
-    uint64_t speculative_walks; /* Bernoulli trials run past the first
-                                   success of their 32-trial chunk (work the
-                                   sequential reference does not do)       */
+    uint64_t speculative_walks; /* Bernoulli trials run past a query's first
+                                   success (work the sequential reference
+                                   does not do; how many depends on timing) */
 } sms_stats;
 
 sms_status sms_stats_read(sms_ctx *ctx, sms_stats *out);

@@ -1127,13 +1127,18 @@ SMS_HD f3 sample_position(const DevScene &sc, const DevShape &s, float sx, float
 enum : int { kPhaseSsFirst = 0, kPhaseSsTrials = 1, kPhaseSsBiased = 2, kPhaseSsWalk = 3, kPhaseMs = 4,
              kPhaseGlints = 5, kPhaseMsWalk = 6, kPhaseGlintWalk = 7, kPhases = 8 };
 
+// trial_jobs .. trial_done of DevCounters: what a launch clears before the
+// first walks of a caster.
+constexpr size_t kTrialStateBytes = 2 * sizeof(unsigned long long) + 2 * sizeof(unsigned int);
+
 struct DevCounters {
     unsigned long long phase_rays[kPhases], phase_nodes[kPhases], phase_tris[kPhases];
     unsigned long long solver_succeeded, solver_failed, bernoulli_calls, bernoulli_iters,
         bernoulli_max, walks, newton_iters, connections, rays, bvh_nodes, tri_tests, speculative_walks;
-    unsigned int trial_count;  // queries appended to the Bernoulli-trial queue
-    unsigned int trial_head;   // next queue entry (must follow trial_count)
-    unsigned int queue_head;   // general persistent-kernel work queue
+    // Bernoulli trials of one caster (TrialState, cleared before its first walks)
+    unsigned long long trial_jobs[2];   // trials drawn from the stream, per pass
+    unsigned int trial_count;  // queries appended to the Bernoulli-trial list
+    unsigned int trial_done;   // of these, queries with a success
     unsigned int error;
 };
 

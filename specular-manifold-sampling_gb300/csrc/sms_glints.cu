@@ -499,8 +499,12 @@ __global__ void __launch_bounds__(128) glint_first_kernel(DevScene sc, SolverCfg
     flush_stats(st, ctr, err, kPhaseGlints);
 }
 
-// Bernoulli trials 32 at a time (:76-105): success when the trial converges
-// within uniqueness_threshold (in uv) of the first glint.
+// Bernoulli trials 32 at a time, a warp per query (:76-105): success when the
+// trial converges within uniqueness_threshold (in uv) of the first glint.  A
+// glint walk is a few hundred instructions, so drawing each trial from the
+// stream of the ray-casting estimators (sms_trials.cuh), with its own query
+// load and emitter sample, costs more than it saves: 976^2 pixels on the 512^2
+// map 118 us against 100 us.
 __global__ void __launch_bounds__(128) glint_trials_kernel(DevScene sc, SolverCfg cfg, const float *__restrict__ qs,
                                                            uint32_t n, uint64_t seed, uint64_t stream_off,
                                                            float *__restrict__ value, int *__restrict__ count,
@@ -512,7 +516,7 @@ __global__ void __launch_bounds__(128) glint_trials_kernel(DevScene sc, SolverCf
     const unsigned n_list = *(volatile unsigned *)&ctr->trial_count;
     while (true) {
         unsigned idx = 0;
-        if (lane == 0) idx = atomicAdd(&ctr->trial_head, 1u);
+        if (lane == 0) idx = (unsigned)atomicAdd(&ctr->trial_jobs[0], 1ull);
         idx = __shfl_sync(kFullG, idx, 0);
         if (idx >= n_list) break;
         uint32_t qi = scr.list[idx];
@@ -637,7 +641,7 @@ cudaError_t launch_glint_connect(const DevScene &sc, const SolverCfg &cfg, const
         if (G == 16) glint_biased_kernel<16><<<blocks, 128, 0, s>>>(sc, cfg, q, n, seed, stream_off, value, count, walks, ctr);
         else glint_biased_kernel<32><<<blocks, 128, 0, s>>>(sc, cfg, q, n, seed, stream_off, value, count, walks, ctr);
     } else {
-        cudaError_t e = cudaMemsetAsync(&ctr->trial_count, 0, 2 * sizeof(unsigned), s);
+        cudaError_t e = cudaMemsetAsync(&ctr->trial_jobs, 0, kTrialStateBytes, s);
         if (e != cudaSuccess) return e;
         glint_first_kernel<<<(n + 127) / 128, 128, 0, s>>>(sc, cfg, q, n, seed, stream_off, value, count, walks, scr,
                                                            ctr);

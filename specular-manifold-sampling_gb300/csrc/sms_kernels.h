@@ -34,8 +34,8 @@ struct SolverCfg {
     // its path and bounce, so that results do not depend on which paths of a
     // wavefront reached a receiver or on how the queries were batched).
     const uint64_t *streams;
-    // Queries a lane group of the Bernoulli-trial kernel claims from the work
-    // queue per atomic (1: one at a time).
+    // Rounds of trials a warp of the Bernoulli-trial kernel claims from the
+    // stream per atomic, at least.
     int queue_chunk;
 };
 

@@ -93,7 +93,7 @@ cudaError_t launch_ms_connect(const DevScene &sc, const SolverCfg &cfg, int boun
         if (e == cudaSuccess) e = cudaMemsetAsync(walks, 0, (size_t)n * sizeof(int), s);
         return e;
     }
-    const int bps = blocks_per_sm > 0 ? blocks_per_sm : 16;
+    const int bps = blocks_per_sm;
     if (sc.ms_rough) {
         // rough chain shapes (offset normals); the host refuses rough + normal-mapped
         if (sc.ms_nm) return cudaErrorNotSupported;

@@ -29,6 +29,7 @@
 #include "sms_device.cuh"
 #include "sms_estimator.cuh"
 #include "sms_kernels.h"
+#include "sms_trials.cuh"
 
 namespace sms {
 
@@ -792,12 +793,12 @@ __global__ void __launch_bounds__(128) ms_first_kernel(DevScene sc, SolverCfg cf
                                                        uint32_t n, uint64_t seed, uint64_t stream_off,
                                                        float *__restrict__ value, int *__restrict__ count,
                                                        int *__restrict__ walks, SsScratch scr, int *__restrict__ tmpl_out,
-                                                       DevCounters *ctr) {
-    uint32_t qi = blockIdx.x * blockDim.x + threadIdx.x;
+                                                       DevCounters *ctr, int lanes) {
+    const uint32_t qi = (blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32) * (uint32_t)lanes + (threadIdx.x & 31);
     LaneStats st;
     uint32_t err = 0;
     bool enqueue = false;
-    if (qi < n) {
+    if ((int)(threadIdx.x & 31) < lanes && qi < n) {
         Query Q = load_query(qs, n, qi);
         Pcg32 rng = query_rng(seed, query_stream(cfg, stream_off, qi), 0);
         Light L;
@@ -863,7 +864,7 @@ __global__ void __launch_bounds__(128) ms_first_kernel(DevScene sc, SolverCfg cf
         value[qi] = acc.x;
         value[(size_t)n + qi] = acc.y;
         value[2 * (size_t)n + qi] = acc.z;
-        count[qi] = 0;
+        count[qi] = enqueue ? kTrialOpen : 0;
         walks[qi] = nw;
     }
     unsigned want = __ballot_sync(kFull, enqueue);
@@ -877,92 +878,66 @@ __global__ void __launch_bounds__(128) ms_first_kernel(DevScene sc, SolverCfg cf
     flush_stats(st, ctr, err, kPhaseMs);
 }
 
-// Part 2: Bernoulli trials, 32 per warp step (:111-135); trial walks must
-// reproduce the template's shapes (and, kRough, scatter about its offsets).
+// Blocks per SM of the trial kernel: what 168 registers (chains of two) let
+// reside.  More blocks with fewer registers lose to spills: 20,011 slab points
+// at 3 / 4 / 5 / 6 / 8 blocks 4.1 / 4.5 / 5.0 / 5.4 / 6.2 ms.
+constexpr int kMsWalkBlocks = 3;
+
+// Part 2: Bernoulli trials (:111-135), one lane per trial, drawn from the
+// stream of sms_trials.cuh; trial walks must reproduce the template's shapes
+// (and, kRough, scatter about its offsets).
 template <int K, bool kNM, bool kRough = false>
 __global__ void __launch_bounds__(128) ms_trials_kernel(DevScene sc, SolverCfg cfg, int ci, const float *__restrict__ qs,
                                                         uint32_t n, uint64_t seed, uint64_t stream_off,
-                                                        float *__restrict__ value, int *__restrict__ count,
-                                                        int *__restrict__ walks, SsScratch scr,
-                                                        const int *__restrict__ tmpl_in, DevCounters *ctr) {
-    const unsigned lane = threadIdx.x & 31;
+                                                        int *__restrict__ count, SsScratch scr,
+                                                        const int *__restrict__ tmpl_in, DevCounters *ctr, int pass) {
+    const int cap = cfg.max_trials > 0 ? cfg.max_trials : kTrialHardLimit;
+    TrialStream ts(*(volatile unsigned *)&ctr->trial_count, cap, pass);
+    if (ts.total == 0) return;
+    __shared__ TrialBuffer bufs[4];
+    TrialBuffer &buf = bufs[threadIdx.x >> 5];
+    constexpr uint32_t kRun = ms_walk_numbers<K, kRough>();
     LaneStats st;
     uint32_t err = 0;
-    const int cap = cfg.max_trials > 0 ? cfg.max_trials : kTrialHardLimit;
     const int caster = sc.casters_ms[ci];
-    const unsigned n_list = *(volatile unsigned *)&ctr->trial_count;
     while (true) {
-        unsigned idx = 0;
-        if (lane == 0) idx = atomicAdd(&ctr->trial_head, 1u);
-        idx = __shfl_sync(kFull, idx, 0);
-        if (idx >= n_list) break;
-        uint32_t qi = scr.list[idx];
-        Query Q = load_query(qs, n, qi);
-        Pcg32 base = query_rng(seed, query_stream(cfg, stream_off, qi), 0);
-        Light L;
-        sample_emitter(sc, sc.emitters_ms, sc.n_emitters_ms, base, Q.x, L);
-        uint32_t pos = scr.pos[qi];
-        f3 dir0 = mk(scr.dir0[qi], scr.dir0[(size_t)n + qi], scr.dir0[2 * (size_t)n + qi]);
-        int tmpl[K];
-        #pragma unroll
-        for (int b = 0; b < K; ++b) tmpl[b] = tmpl_in[(size_t)b * n + qi];
-        f3 toff[K];
-        float tpdf = 1.f;
-        #pragma unroll
-        for (int b = 0; b < K; ++b) toff[b] = mk(0.f, 0.f, 1.f);
-        if constexpr (kRough) {
-            const float *orow = ms_offset_rows(const_cast<int *>(tmpl_in), n);
+        uint32_t qi;
+        int t;
+        const bool have = ts.next(buf, scr.list, count, ctr, pass, cfg.queue_chunk, qi, t);
+        if (!__any_sync(kFull, have)) break;
+        if (have) {
+            const Query Q = load_query(qs, n, qi);
+            Pcg32 rng = query_rng(seed, query_stream(cfg, stream_off, qi), 0);
+            Light L;
+            sample_emitter(sc, sc.emitters_ms, sc.n_emitters_ms, rng, Q.x, L);
+            const uint32_t pos = scr.pos[qi];
+            int tmpl[K];
             #pragma unroll
-            for (int b = 0; b < K; ++b)
-                toff[b] = mk(orow[(size_t)(3 * b) * n + qi], orow[(size_t)(3 * b + 1) * n + qi],
-                             orow[(size_t)(3 * b + 2) * n + qi]);
-            tpdf = orow[(size_t)(3 * kMaxBounces) * n + qi];
-        }
-        constexpr uint32_t kRun = ms_walk_numbers<K, kRough>();
-        int first = 0;
-        for (int t0 = 1; t0 <= cap; t0 += 32) {
-            int t = t0 + (int)lane;
-            bool succ = false;
+            for (int b = 0; b < K; ++b) tmpl[b] = tmpl_in[(size_t)b * n + qi];
+            f3 toff[K];
+            #pragma unroll
+            for (int b = 0; b < K; ++b) toff[b] = mk(0.f, 0.f, 1.f);
+            if constexpr (kRough) {
+                const float *orow = ms_offset_rows(const_cast<int *>(tmpl_in), n);
+                #pragma unroll
+                for (int b = 0; b < K; ++b)
+                    toff[b] = mk(orow[(size_t)(3 * b) * n + qi], orow[(size_t)(3 * b + 1) * n + qi],
+                                 orow[(size_t)(3 * b + 2) * n + qi]);
+            }
+            rng.advance((uint64_t)(pos - 3u) + kRun * (uint64_t)(t - 1));
+            float sx = rng.next_f32(), sy = rng.next_f32();
+            f3 x1 = sample_position(sc, sc.shapes[caster], sx, sy);
+            Chain<K> c;
             int it = 0;
-            if (t <= cap) {
-                Pcg32 rng = base;
-                rng.advance((uint64_t)(pos - 3u) + kRun * (uint64_t)(t - 1));
-                float sx = rng.next_f32(), sy = rng.next_f32();
-                f3 x1 = sample_position(sc, sc.shapes[caster], sx, sy);
-                Chain<K> c;
-                ChainOffsets<K> co;
-                co.offs = toff;
-                bool ok = seed_chain<K, kNM, kRough>(sc, cfg, caster, Q.x, x1, L.p, tmpl, c, nullptr, err, st, co) &&
-                          chain_newton<K, kNM, kRough>(sc, cfg, Q.x, L.p, tmpl, c, it, err, st,
-                                                       kRough ? toff : nullptr);
-                succ = ok && fabsf(dot(dir0, normalize(c.v[0].p - Q.x)) - 1.f) < cfg.uniqueness_threshold;
+            ChainOffsets<K> co;
+            co.offs = toff;
+            bool succ = seed_chain<K, kNM, kRough>(sc, cfg, caster, Q.x, x1, L.p, tmpl, c, nullptr, err, st, co) &&
+                        chain_newton<K, kNM, kRough>(sc, cfg, Q.x, L.p, tmpl, c, it, err, st, kRough ? toff : nullptr);
+            if (succ) {
+                const f3 dir0 = mk(scr.dir0[qi], scr.dir0[(size_t)n + qi], scr.dir0[2 * (size_t)n + qi]);
+                succ = fabsf(dot(dir0, normalize(c.v[0].p - Q.x)) - 1.f) < cfg.uniqueness_threshold;
             }
-            unsigned b = __ballot_sync(kFull, succ);
-            int f = b ? t0 + __ffs(b) - 1 : 0x7fffffff;
-            if (t <= cap) {
-                if (t <= f) { st.walks++; st.newton += (unsigned)it; }
-                else st.spec++;
-            }
-            if (b) { first = f; break; }
-        }
-        if (lane == 0) {
-            int iterations = first ? first : cap + 1;
-            float inv_prob = first ? (float)first : 0.f;
-            int trial_walks = first ? first : cap;
-            if (!first && cfg.max_trials <= 0) err |= kErrTrialLimit;
-            f3 val = mk(scr.val[qi], scr.val[(size_t)n + qi], scr.val[2 * (size_t)n + qi]);
-            f3 cur = val * inv_prob;
-            // result += value / m_offset_normals_pdf (:198)
-            if (kRough) cur = mk(cur.x / tpdf, cur.y / tpdf, cur.z / tpdf);
-            value[qi] += cur.x;
-            value[(size_t)n + qi] += cur.y;
-            value[2 * (size_t)n + qi] += cur.z;
-            count[qi] = first ? iterations : -1;
-            walks[qi] += trial_walks;
-            scr.pos[qi] = pos + kRun * (uint32_t)trial_walks;
-            st.calls++;
-            st.iters += (unsigned long long)iterations;
-            st.imax = max(st.imax, (unsigned long long)iterations);
+            trial_end(count, ctr, qi, t, succ, it, st);
         }
     }
     flush_stats(st, ctr, err, kPhaseMs);
@@ -993,7 +968,7 @@ cudaError_t ms_connect_k(const DevScene &sc, const SolverCfg &cfg, const float *
     if (cfg.biased) {
         const int G = cfg.max_trials <= 16 ? 16 : 32;
         const uint32_t gpb = 128 / G;
-        uint32_t blocks = std::min<uint32_t>((n + gpb - 1) / gpb, (uint32_t)(num_sms * bps));
+        uint32_t blocks = std::min<uint32_t>((n + gpb - 1) / gpb, (uint32_t)(num_sms * (bps > 0 ? bps : 16)));
         phase_begin(tm, kPhaseMs, s);
         auto kernel = G == 16 ? ms_biased_kernel<K, 16, kNM, kRough> : ms_biased_kernel<K, 32, kNM, kRough>;
         kernel<<<blocks, 128, 0, s>>>(sc, cfg, q, n, seed, stream_off, value, count, walks, ctr);
@@ -1001,14 +976,22 @@ cudaError_t ms_connect_k(const DevScene &sc, const SolverCfg &cfg, const float *
         return cudaGetLastError();
     }
     for (int c = 0; c < sc.n_casters_ms; ++c) {
-        cudaError_t e = cudaMemsetAsync(&ctr->trial_count, 0, 2 * sizeof(unsigned), s);
+        cudaError_t e = cudaMemsetAsync(&ctr->trial_jobs, 0, kTrialStateBytes, s);
         if (e != cudaSuccess) return e;
         phase_begin(tm, kPhaseMs, s);
         auto first = ms_first_kernel<K, kNM, kRough>;
         auto trials = ms_trials_kernel<K, kNM, kRough>;
-        first<<<(n + 127) / 128, 128, 0, s>>>(sc, cfg, c, q, n, seed, stream_off, value, count, walks, scr, tmpl, ctr);
-        trials<<<num_sms * bps, 128, 0, s>>>(sc, cfg, c, q, n, seed, stream_off, value, count, walks, scr, tmpl,
-                                              ctr);
+        const int lanes = first_walk_lanes(n, num_sms);
+        first<<<first_walk_blocks(n, lanes), 128, 0, s>>>(sc, cfg, c, q, n, seed, stream_off, value, count, walks, scr, tmpl, ctr, lanes);
+        const int tblocks = num_sms * (bps > 0 ? bps : kMsWalkBlocks);
+        const int cap = cfg.max_trials > 0 ? cfg.max_trials : kTrialHardLimit;
+        for (int pass = trial_split_possible(n, cap, tblocks) ? 0 : 1; pass < 2; ++pass)
+            trials<<<tblocks, 128, 0, s>>>(sc, cfg, c, q, n, seed, stream_off, count, scr, tmpl, ctr, pass);
+        // result += value / m_offset_normals_pdf (:198)
+        const float *pdf = kRough ? reinterpret_cast<const float *>(tmpl + (size_t)kMaxBounces * n) +
+                                        (size_t)(3 * kMaxBounces) * n : nullptr;
+        trials_finish_kernel<<<finish_blocks(n, num_sms), 128, 0, s>>>(
+            n, value, count, walks, scr, pdf, cap, cfg.max_trials <= 0, ms_walk_numbers<K, kRough>(), kPhaseMs, ctr);
         phase_end(tm, s);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;

@@ -21,11 +21,12 @@
 //                       first walk, the light visibility test and the
 //                       contribution; queries that need Bernoulli trials are
 //                       appended to a device work queue.
-//   ss_trials_kernel    unbiased estimator, part 2 (:111-135): persistent warps
-//                       take queries from the queue and run the Bernoulli
-//                       trials 32 at a time (lane = trial); the first success is
-//                       found by ballot, so one query's trials never serialize
-//                       on a single lane.
+//   ss_trials_kernel    unbiased estimator, part 2 (:111-135): the Bernoulli
+//                       trials of all queued queries as one stream, one lane
+//                       per trial (sms_trials.cuh); the smallest successful
+//                       trial of each query stands in count, so one query's
+//                       trials never serialize on a lane or a warp.
+//   trials_finish_kernel  part 3: value, counts and statistics from them.
 #include <algorithm>
 
 #include "sms_device.cuh"
@@ -265,18 +266,18 @@ cudaError_t launch_ss_connect(const DevScene &sc, const SolverCfg &cfg, const fl
         return e;
     }
     for (int c = 0; c < sc.n_casters_ss; ++c) {
-        cudaError_t e = cudaMemsetAsync(&ctr->trial_count, 0, 2 * sizeof(unsigned), s);
+        cudaError_t e = cudaMemsetAsync(&ctr->trial_jobs, 0, kTrialStateBytes, s);
         if (e != cudaSuccess) return e;
         const int var = ss_variant(sc, cfg, c);
         if (var & 4)
             e = launch_ss_caster_nm(var, sc, cfg, c, q, n, seed, stream_off, value, count, walks, ctr, scr, num_sms,
-                                    bps, tm, s, trial_group);
+                                    blocks_per_sm, tm, s, trial_group);
         else if (var)
             e = ss_caster_launch<1, true>(sc, cfg, c, q, n, seed, stream_off, value, count, walks, ctr, scr, num_sms,
-                                          bps, tm, s, prop, trial_group, treelet);
+                                          blocks_per_sm, tm, s, prop, trial_group, treelet);
         else
             e = ss_caster_launch<0, true>(sc, cfg, c, q, n, seed, stream_off, value, count, walks, ctr, scr, num_sms,
-                                          bps, tm, s, prop, trial_group, treelet);
+                                          blocks_per_sm, tm, s, prop, trial_group, treelet);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;

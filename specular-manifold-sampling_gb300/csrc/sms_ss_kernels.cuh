@@ -17,6 +17,7 @@
 #include "sms_estimator.cuh"
 #include "sms_kernels.h"
 #include "sms_mlp.cuh"
+#include "sms_trials.cuh"
 
 namespace sms {
 
@@ -30,8 +31,8 @@ namespace sms {
 #endif
 // Normal-mapped casters: the map's frame and the two-stage solver add
 // arithmetic, not traversal, so what counts is that the step stays in
-// registers.  4 blocks (128 registers); normal-mapped pane with the
-// two-stage solver at 4 and 9 blocks: 0.69 and 0.83 ms (15,203 points, conductor).
+// registers.  4 blocks (128 registers); pane of 30,000 points with the
+// two-stage solver at 4 / 5 / 6 / 9 blocks: 0.76 / 0.80 / 0.91 / 1.06 ms.
 constexpr int ss_walk_blocks(int var) { return (var & 4) ? 4 : SMS_SS_WALK_MIN_BLOCKS; }
 
 // ------------------------------------------------------ biased estimator
@@ -167,11 +168,11 @@ __global__ void __launch_bounds__(128, ss_walk_blocks(kVar)) ss_first_kernel(Dev
                                                        uint32_t n, uint64_t seed, uint64_t stream_off,
                                                        float *__restrict__ value, int *__restrict__ count,
                                                        int *__restrict__ walks, SsScratch scr, DevCounters *ctr,
-                                                       mlp::SeedProposal pr) {
+                                                       mlp::SeedProposal pr, int lanes) {
     constexpr bool kRough = (kVar & 1) != 0, kTwo = (kVar & 2) != 0, kNM = (kVar & 4) != 0;
-    const uint32_t qi = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = qi < n;
     const unsigned lane = threadIdx.x & 31;
+    const uint32_t qi = (blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32) * (uint32_t)lanes + lane;
+    const bool active = (int)lane < lanes && qi < n;
     LaneStats st;
     uint32_t err = 0;
     bool enqueue = false;
@@ -245,7 +246,7 @@ __global__ void __launch_bounds__(128, ss_walk_blocks(kVar)) ss_first_kernel(Dev
         value[qi] = acc.x;
         value[(size_t)n + qi] = acc.y;
         value[2 * (size_t)n + qi] = acc.z;
-        count[qi] = 0;
+        count[qi] = enqueue ? kTrialOpen : 0;
         walks[qi] = nw;
     }
     // warp-aggregated append to the trial queue
@@ -261,89 +262,48 @@ __global__ void __launch_bounds__(128, ss_walk_blocks(kVar)) ss_first_kernel(Dev
 }
 
 // ------------------------------------------------ unbiased: Bernoulli trials
-// Persistent warps split into groups of G lanes; each group takes queries
-// from the queue and runs their Bernoulli trials G at a time (lane = trial).
 // For query q with first-walk direction dir0 the trials are t = 1, 2, ...;
 // trial t draws stream positions pos + S(t-1) .. (S = 2 draws per walk, 3 with
-// a learned proposal), so the first success -- found by ballot -- is exactly
-// the reference's sequential trial count (manifold_ss.cpp:115-135) whatever
-// G is.  G = 32 suits uniform seeding (tens of trials per query); a learned
-// proposal succeeds within a few trials and runs G = 8 (four queries per warp)
-// to cut the speculative walks past the first success.  Every trial redraws
-// its seed from the same per-query proposal as the first walk, so the count
-// still estimates the inverse probability of reaching dir0.
-//
-// All lanes run one warp-uniform loop: groups whose query finished fetch the
-// next one at the top, so every ballot and shuffle has the whole warp.
-template <bool kLearned, int G, int kVar, bool kTree = false>
+// a learned proposal), so the smallest successful t is exactly the reference's
+// sequential trial count (manifold_ss.cpp:115-135), whichever trials ran side
+// by side.  Every trial redraws its seed from the same per-query proposal as
+// the first walk, so the count still estimates the inverse probability of
+// reaching dir0.  One lane per trial, drawn from the stream of sms_trials.cuh.
+template <bool kLearned, int kVar, bool kTree = false>
 __global__ void __launch_bounds__(128, ss_walk_blocks(kVar)) ss_trials_kernel(DevScene sc, SolverCfg cfg, int c, const float *__restrict__ qs,
                                                         uint32_t n, uint64_t seed, uint64_t stream_off,
-                                                        float *__restrict__ value, int *__restrict__ count,
-                                                        int *__restrict__ walks, SsScratch scr, DevCounters *ctr,
-                                                        mlp::SeedProposal pr) {
-    static_assert(G == 8 || G == 16 || G == 32, "group size");
+                                                        int *__restrict__ count, SsScratch scr, DevCounters *ctr,
+                                                        mlp::SeedProposal pr, int pass, int lanes) {
     constexpr bool kRough = (kVar & 1) != 0, kTwo = (kVar & 2) != 0, kNM = (kVar & 4) != 0;
+    const int cap = cfg.max_trials > 0 ? cfg.max_trials : kTrialHardLimit;
+    TrialStream ts(*(volatile unsigned *)&ctr->trial_count, cap, pass, lanes);
+    if (ts.total == 0) return;
     if (kTree) tree_smem_fill(sc);
-    const unsigned full = 0xffffffffu;
-    const unsigned lane = threadIdx.x & 31;
-    const unsigned gbase = lane & ~(unsigned)(G - 1), gl = lane - gbase;
-    const unsigned gmask = (G == 32) ? full : (((1u << G) - 1u) << gbase);
+    __shared__ TrialBuffer bufs[4];
+    TrialBuffer &buf = bufs[threadIdx.x >> 5];
     constexpr uint32_t kStride = (kLearned ? 3u : 2u) + (kTwo ? 2u : 0u);   // numbers per walk
     LaneStats st;
     uint32_t err = 0;
-    const int cap = cfg.max_trials > 0 ? cfg.max_trials : kTrialHardLimit;
     const int caster = sc.casters_ss[c];
-    const unsigned n_list = *(volatile unsigned *)&ctr->trial_count;
-    // per-group state (replicated on the group's lanes)
-    bool have = false, drained = false;
-    const unsigned chunk = cfg.queue_chunk > 1 ? (unsigned)cfg.queue_chunk : 1u;
-    unsigned cnext = 0, cend = 0;   // the group's claimed range of the queue
-    uint32_t qi = 0, pos = 0;
-    int t0 = 1;
-    Query Q;
-    Light L;
-    Pcg32 base;
-    f3 dir0 = splat(0.f);
-    f3 no = mk(0.f, 0.f, 1.f);
-    const DevShape &cshape = sc.shapes[caster];
     while (true) {
-        // groups without a query take the next one, claiming `chunk` queue
-        // entries per atomic
-        const bool need = !have && !drained;
-        const bool claim = need && cnext == cend;
-        unsigned got = 0;
-        if (claim && gl == 0) got = atomicAdd(&ctr->trial_head, chunk);
-        got = __shfl_sync(full, got, gbase);
-        if (claim) { cnext = got; cend = got + chunk; }
-        const unsigned idx = cnext;
-        if (need) {
-            ++cnext;
-            if (idx < n_list) {
-                have = true;
-                qi = scr.list[idx];
-                Q = load_query(qs, n, qi);
-                base = query_rng(seed, query_stream(cfg, stream_off, qi), 0);
-                sample_emitter(sc, sc.emitters_ss, sc.n_emitters_ss, base, Q.x, L);   // base sits at position 3
-                pos = scr.pos[qi];
-                dir0 = mk(scr.dir0[qi], scr.dir0[(size_t)n + qi], scr.dir0[2 * (size_t)n + qi]);
-                t0 = 1;
-                if (kRough) {
-                    // the offset normal drawn before the first walk
-                    Pcg32 r0 = base;
-                    r0.advance((uint64_t)(pos - 3u - kStride - 2u));
-                    float p_off;
-                    no = caster_offset(cshape, r0, p_off);
-                }
-            } else {
-                drained = true;
+        uint32_t qi;
+        int t;
+        const bool have = ts.next(buf, scr.list, count, ctr, pass, cfg.queue_chunk, qi, t);
+        if (!__any_sync(0xffffffffu, have)) break;
+        if (have) {
+            const Query Q = load_query(qs, n, qi);
+            Pcg32 rng = query_rng(seed, query_stream(cfg, stream_off, qi), 0);
+            Light L;
+            sample_emitter(sc, sc.emitters_ss, sc.n_emitters_ss, rng, Q.x, L);   // rng sits at position 3
+            const uint32_t pos = scr.pos[qi];
+            f3 no = mk(0.f, 0.f, 1.f);
+            if (kRough) {
+                // the offset normal drawn before the first walk
+                Pcg32 r0 = rng;
+                r0.advance((uint64_t)(pos - 3u - kStride - 2u));
+                float p_off;
+                no = caster_offset(sc.shapes[caster], r0, p_off);
             }
-        }
-        if (__ballot_sync(full, have) == 0u) break;
-        const int t = t0 + (int)gl;
-        bool succ = false;
-        int it = 0;
-        if (have && t <= cap) {
-            Pcg32 rng = base;
             rng.advance((uint64_t)(pos - 3u) + kStride * (uint64_t)(t - 1));
             f3 sp;
             if constexpr (kLearned) {
@@ -356,47 +316,14 @@ __global__ void __launch_bounds__(128, ss_walk_blocks(kVar)) ss_trials_kernel(De
             float g0 = 0.f, g1 = 0.f;
             if (kTwo) { g0 = rng.next_f32(); g1 = rng.next_f32(); }
             Vtx v;
-            succ = ss_walk<kRough, kTwo, kNM, kTree>(sc, cfg, caster, Q.x, L.p, sp, v, it, err, st, nullptr, no, g0,
-                                                     g1) &&
-                   fabsf(dot(dir0, normalize(v.p - Q.x)) - 1.f) < cfg.uniqueness_threshold;
-        }
-        const unsigned b = (__ballot_sync(full, succ) & gmask) >> gbase;
-        const int f = b ? t0 + __ffs(b) - 1 : 0x7fffffff;
-        if (have && t <= cap) {
-            // trials up to the first success are the reference's walks; the
-            // rest of the chunk is speculative work
-            if (t <= f) { st.walks++; st.newton += (unsigned)it; }
-            else st.spec++;
-        }
-        if (have && (b || t0 + G > cap)) {
-            if (gl == 0) {
-                float inv_prob;
-                int iterations, trial_walks;
-                if (b) {
-                    iterations = f;
-                    inv_prob = (float)f;
-                    trial_walks = f;
-                } else {
-                    iterations = cap + 1;
-                    inv_prob = 0.f;
-                    trial_walks = cap;
-                    if (cfg.max_trials <= 0) err |= kErrTrialLimit;
-                }
-                f3 val = mk(scr.val[qi], scr.val[(size_t)n + qi], scr.val[2 * (size_t)n + qi]);
-                f3 cur = val * inv_prob;
-                value[qi] += cur.x;
-                value[(size_t)n + qi] += cur.y;
-                value[2 * (size_t)n + qi] += cur.z;
-                count[qi] = b ? iterations : -1;
-                walks[qi] += trial_walks;
-                scr.pos[qi] = pos + kStride * (uint32_t)trial_walks;
-                st.calls++;
-                st.iters += (unsigned long long)iterations;
-                st.imax = max(st.imax, (unsigned long long)iterations);
+            int it;
+            bool succ = ss_walk<kRough, kTwo, kNM, kTree>(sc, cfg, caster, Q.x, L.p, sp, v, it, err, st, nullptr, no,
+                                                          g0, g1);
+            if (succ) {
+                const f3 dir0 = mk(scr.dir0[qi], scr.dir0[(size_t)n + qi], scr.dir0[2 * (size_t)n + qi]);
+                succ = fabsf(dot(dir0, normalize(v.p - Q.x)) - 1.f) < cfg.uniqueness_threshold;
             }
-            have = false;
-        } else if (have) {
-            t0 += G;
+            trial_end(count, ctr, qi, t, succ, it, st);
         }
     }
     flush_stats(st, ctr, err, kPhaseSsTrials);
@@ -434,48 +361,41 @@ cudaError_t ss_caster_launch(const DevScene &sc, const SolverCfg &cfg, int c, co
     const mlp::SeedProposal pr = learned ? *prop : mlp::SeedProposal{};
     phase_begin(tm, kPhaseSsFirst, s);
     cudaError_t e = cudaSuccess;
+    const int lanes = first_walk_lanes(n, num_sms);
+    const uint32_t fblocks = first_walk_blocks(n, lanes);
     if constexpr (kLearnedOk) {
         if (learned) {
             e = launch_ss_proposal(sc, cfg, q, n, seed, stream_off, pr, num_sms, s);
             if (e != cudaSuccess) return e;
-            ss_first_kernel<true, kVar><<<(n + 127) / 128, 128, 0, s>>>(sc, cfg, c, q, n, seed, stream_off, value,
-                                                                        count, walks, scr, ctr, pr);
+            ss_first_kernel<true, kVar><<<fblocks, 128, 0, s>>>(sc, cfg, c, q, n, seed, stream_off, value, count,
+                                                                walks, scr, ctr, pr, lanes);
         }
     }
     if (!learned)
-        ss_first_kernel<false, kVar><<<(n + 127) / 128, 128, 0, s>>>(sc, cfg, c, q, n, seed, stream_off, value,
-                                                                     count, walks, scr, ctr, pr);
+        ss_first_kernel<false, kVar><<<fblocks, 128, 0, s>>>(sc, cfg, c, q, n, seed, stream_off, value, count, walks,
+                                                             scr, ctr, pr, lanes);
     phase_end(tm, s);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     phase_begin(tm, kPhaseSsTrials, s);
-    const int group = trial_group > 0 ? trial_group : (learned ? 8 : 32);
+    auto trials = ss_trials_kernel<false, kVar>;
+    if constexpr ((kVar & 4) == 0) {   // the treelet serves the plain and rough casters
+        if (st.n_tnodes) trials = ss_trials_kernel<false, kVar, true>;
+    }
     if constexpr (kLearnedOk) {
-        if (learned) {
-            auto trials = group == 8 ? ss_trials_kernel<true, 8, kVar>
-                          : group == 16 ? ss_trials_kernel<true, 16, kVar> : ss_trials_kernel<true, 32, kVar>;
-            if constexpr ((kVar & 4) == 0) {   // the treelet serves the plain and rough casters
-                if (st.n_tnodes)
-                    trials = group == 8 ? ss_trials_kernel<true, 8, kVar, true>
-                             : group == 16 ? ss_trials_kernel<true, 16, kVar, true>
-                                           : ss_trials_kernel<true, 32, kVar, true>;
-            }
-            trials<<<num_sms * bps, 128, tsmem, s>>>(st, cfg, c, q, n, seed, stream_off, value, count, walks, scr, ctr,
-                                                     pr);
-        }
-    }
-    if (!learned) {
-        auto trials = group == 8 ? ss_trials_kernel<false, 8, kVar>
-                      : group == 16 ? ss_trials_kernel<false, 16, kVar> : ss_trials_kernel<false, 32, kVar>;
+        if (learned) trials = ss_trials_kernel<true, kVar>;
         if constexpr ((kVar & 4) == 0) {
-            if (st.n_tnodes)
-                trials = group == 8 ? ss_trials_kernel<false, 8, kVar, true>
-                         : group == 16 ? ss_trials_kernel<false, 16, kVar, true>
-                                       : ss_trials_kernel<false, 32, kVar, true>;
+            if (learned && st.n_tnodes) trials = ss_trials_kernel<true, kVar, true>;
         }
-        trials<<<num_sms * bps, 128, tsmem, s>>>(st, cfg, c, q, n, seed, stream_off, value, count, walks, scr, ctr,
-                                                 pr);
     }
+    const int tblocks = num_sms * (bps > 0 ? bps : ss_walk_blocks(kVar));
+    const int cap = cfg.max_trials > 0 ? cfg.max_trials : kTrialHardLimit;
+    for (int pass = trial_split_possible(n, cap, tblocks) ? 0 : 1; pass < 2; ++pass)
+        trials<<<tblocks, 128, tsmem, s>>>(st, cfg, c, q, n, seed, stream_off, count, scr, ctr, pr, pass,
+                                           trial_group > 0 ? trial_group : 32);
+    const uint32_t stride = (learned ? 3u : 2u) + ((kVar & 2) ? 2u : 0u);
+    trials_finish_kernel<<<finish_blocks(n, num_sms), 128, 0, s>>>(n, value, count, walks, scr, nullptr, cap,
+                                                                   cfg.max_trials <= 0, stride, kPhaseSsTrials, ctr);
     phase_end(tm, s);
     return cudaGetLastError();
 }

@@ -1,0 +1,224 @@
+// sms_trials.cuh -- scheduling of the unbiased estimators' Bernoulli trials.
+//
+// After the first walks, n_list queries wait for trials t = 1, 2, ... until
+// the first success or the cap.  A trial is a walk of its own with its own run
+// of random numbers, so any number of a query's trials can run at once; the
+// answer is the smallest successful t, which count[q] holds while the trials
+// run (kTrialOpen: none yet).  The trials form one stream in trial-major
+// order -- every open query's t before anyone's t + 1 -- that the warps of a
+// persistent grid consume lane by lane; a trial whose query is known to
+// succeed earlier is dropped when it is drawn.  Large lists thus run few
+// trials past a success (about lanes / n_list per query), and short lists
+// spread over the whole chip: the last query's 256 trials are 256 lanes' work
+// in one go instead of eight 32-trial rounds of one warp.
+//
+// What it costs is trials past a success: up to the grid's lanes / n_list per
+// query.  Holding a query to 32 or 64 trials in flight was slower (points of the
+// 512^2 water, GB300; one warp per query with 32 trials at a time before):
+//   points             before    32     64    no limit
+//   32,003              6.5 ms   3.6    3.3    3.2
+//   7,321 (64^2, 100)   2.2      1.25   1.1    0.84
+//   300 (host)          3.5      0.59   0.59   0.59
+// (1M points: 40.5 -> 36.8 ms.)
+//
+// Between the two, a list shorter than the grid would still launch dozens of
+// trials per query at once although most succeed at their first (a flat
+// caster: 1.4 trials a query): pass 0 then runs t = 1 alone and pass 1 the
+// rest.
+#pragma once
+#include "sms_device.cuh"
+#include "sms_estimator.cuh"
+
+namespace sms {
+
+constexpr int kTrialOpen = 0x7fffffff;
+// Lists of at most this many grids' worth of trials run in a single pass.  A
+// pass of first trials costs one walk's latency (0.25 ms); what it saves is the
+// speculative trials of the queries that succeed at once.  Pane of 30,000
+// points (15,153 listed, 64 trials, 5.5 grids of 9 blocks per SM): one pass
+// 1.07 ms, two passes 1.34 ms; slab of 20,011 points (14,529 listed, 128
+// trials, 32 grids of 3 blocks): two passes 4.0 ms, one pass 4.5 ms.
+constexpr unsigned kTrialSinglePass = 16;
+
+// Trials [lo, hi] of one pass, and the lanes of a warp that take part (`most`
+// at most): fewer when all of the pass's trials fit the grid that way (lanes
+// of one warp wait for each other's rays).
+struct TrialPlan {
+    int lo, hi;
+    int lanes;
+};
+
+SMS_D TrialPlan trial_plan(unsigned n_list, int cap, int pass, int most) {
+    const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x / 32), all = 32ull * warps;
+    const unsigned long long jobs = (unsigned long long)n_list * (unsigned)cap;
+    const bool split = n_list < all && jobs > kTrialSinglePass * all;
+    TrialPlan p;
+    p.lo = 1;
+    p.hi = cap;
+    if (pass == 0) p.hi = split ? 1 : 0;
+    else if (split) p.lo = 2;
+    const unsigned long long mine = (unsigned long long)n_list * (unsigned)max(0, p.hi - p.lo + 1);
+    p.lanes = (int)min((unsigned long long)most, max(1ull, (mine + warps - 1) / warps));
+    return p;
+}
+
+// A warp's end of the stream: a claimed range of the pass's trial indices and
+// the drawn trials that wait for a lane.
+struct TrialBuffer {
+    uint32_t qi[64];
+    int t[64];
+};
+
+struct TrialStream {
+    unsigned long long cur = 0, end = 0;   // claimed range
+    unsigned long long total;
+    unsigned n_list;
+    TrialPlan plan;
+    int ready = 0;       // buffered trials
+    bool drained = false;
+
+    SMS_D TrialStream(unsigned n, int cap, int pass, int most = 32) : n_list(n), plan(trial_plan(n, cap, pass, most)) {
+        total = (unsigned long long)n * (unsigned)max(0, plan.hi - plan.lo + 1);
+    }
+
+    // Up to plan.lanes trials for lanes 0 .. k-1, in stream order; returns
+    // whether this lane has one.  Called by the whole warp.  false for every
+    // lane: the pass is done.
+    SMS_D bool next(TrialBuffer &buf, const uint32_t *list, const int *count, DevCounters *ctr, int pass,
+                    int chunk, uint32_t &qi, int &t) {
+        const unsigned full = 0xffffffffu;
+        const int lane = (int)(threadIdx.x & 31);
+        while (ready < plan.lanes && !drained) {
+            if (cur >= end) {
+                // a claim is a few rounds of the warp (chunk at least), but no
+                // more than its share of the stream
+                const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x / 32);
+                const unsigned long long share = total / (4 * warps) / plan.lanes;
+                const unsigned claim = (unsigned)plan.lanes * (unsigned)max((unsigned long long)chunk, min(4ull, max(1ull, share)));
+                unsigned long long got = 0;
+                unsigned done = 0;
+                if (lane == 0) {
+                    got = atomicAdd(&ctr->trial_jobs[pass], (unsigned long long)claim);
+                    done = *(volatile unsigned *)&ctr->trial_done;
+                }
+                cur = __shfl_sync(full, got, 0);
+                done = __shfl_sync(full, done, 0);
+                end = min(cur + claim, total);
+                if (cur >= total || done >= n_list) { drained = true; break; }
+            }
+            const int k = (int)min((unsigned long long)plan.lanes, end - cur);
+            bool open = false;
+            uint32_t q = 0;
+            int tt = 0;
+            if (lane < k) {
+                const unsigned long long j = cur + (unsigned)lane;
+                const unsigned long long row = (j >> 32) == 0 ? (unsigned)j / n_list : j / n_list;
+                tt = plan.lo + (int)row;
+                q = list[(unsigned)(j - row * n_list)];
+                open = *(volatile const int *)(count + q) > tt;
+            }
+            const unsigned m = __ballot_sync(full, open);
+            if (open) {
+                const int at = ready + __popc(m & ((1u << lane) - 1u));
+                buf.qi[at] = q;
+                buf.t[at] = tt;
+            }
+            ready += __popc(m);
+            cur += (unsigned)k;
+        }
+        __syncwarp();
+        const int take = min(ready, plan.lanes);
+        const bool mine = lane < take;
+        if (mine) { qi = buf.qi[lane]; t = buf.t[lane]; }
+        // what is left moves to the front (at most plan.lanes - 1 entries)
+        uint32_t q2 = 0;
+        int t2 = 0;
+        const bool move = take + lane < ready;
+        if (move) { q2 = buf.qi[take + lane]; t2 = buf.t[take + lane]; }
+        __syncwarp();
+        if (move) { buf.qi[lane] = q2; buf.t[lane] = t2; }
+        ready -= take;
+        __syncwarp();
+        return mine;
+    }
+};
+
+// Record the end of trial t of query qi.
+SMS_D void trial_end(int *count, DevCounters *ctr, uint32_t qi, int t, bool succ, int it, LaneStats &st) {
+    st.spec++;   // the trials up to each query's first success are taken out at the end
+    if (succ) {
+        if (atomicMin(count + qi, t) == kTrialOpen) atomicAdd(&ctr->trial_done, 1u);
+        st.newton += (unsigned)it;
+    } else if (*(volatile const int *)(count + qi) > t) {
+        st.newton += (unsigned)it;
+    }
+}
+
+// The estimate's trial statistics once all trials have run: f the first
+// success or kTrialOpen.
+SMS_D void trial_stats(int f, int cap, bool unbounded, uint32_t &err, LaneStats &st) {
+    const bool found = f != kTrialOpen;
+    const unsigned long long w = (unsigned long long)(found ? f : cap);
+    if (!found && unbounded) err |= kErrTrialLimit;
+    st.walks += w;
+    st.spec -= w;
+    st.calls++;
+    st.iters += found ? w : w + 1;
+    st.imax = max(st.imax, found ? w : w + 1);
+}
+
+// A result of n_list queries after their trials: value += first-walk
+// contribution x trial count (over the template's offset density pdf, where
+// given), the query's stream position behind its trials.
+static __global__ void __launch_bounds__(128) trials_finish_kernel(uint32_t n, float *__restrict__ value,
+                                                                   int *__restrict__ count, int *__restrict__ walks,
+                                                                   SsScratch scr, const float *__restrict__ pdf,
+                                                                   int cap, int unbounded, uint32_t stride, int phase,
+                                                                   DevCounters *ctr) {
+    LaneStats st;
+    uint32_t err = 0;
+    const unsigned n_list = *(volatile unsigned *)&ctr->trial_count;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n_list; i += gridDim.x * blockDim.x) {
+        const uint32_t qi = scr.list[i];
+        const int f = count[qi];
+        const bool found = f != kTrialOpen;
+        const float inv_prob = found ? (float)f : 0.f;
+        const int trial_walks = found ? f : cap;
+        trial_stats(f, cap, unbounded != 0, err, st);
+        f3 cur = mk(scr.val[qi], scr.val[(size_t)n + qi], scr.val[2 * (size_t)n + qi]) * inv_prob;
+        if (pdf) cur = mk(cur.x / pdf[qi], cur.y / pdf[qi], cur.z / pdf[qi]);
+        value[qi] += cur.x;
+        value[(size_t)n + qi] += cur.y;
+        value[2 * (size_t)n + qi] += cur.z;
+        count[qi] = found ? f : -1;
+        walks[qi] += trial_walks;
+        scr.pos[qi] += stride * (uint32_t)trial_walks;
+    }
+    flush_stats(st, ctr, err, phase);
+}
+
+// Lanes of a warp that run first walks, one query each.  Lanes of one warp
+// wait for each other's rays, so a batch below kFirstWarps full warps per SM
+// (two per scheduler, enough to hide each other's latency) takes that many
+// warps with fewer queries each: 300 points 0.67 -> 0.20 ms; spread over all
+// resident warps instead, larger batches lose to the extra instructions (pane
+// of 30,000 points, 32 / 25 / 6 queries a warp: 0.19 / 0.19 / 0.44 ms).
+constexpr int kFirstWarps = 8;
+inline int first_walk_lanes(uint32_t n, int num_sms) {
+    const uint32_t warps = (uint32_t)(num_sms * kFirstWarps), l = n / warps + (n % warps != 0);
+    return (int)(l < 1 ? 1 : l > 32 ? 32 : l);
+}
+inline uint32_t first_walk_blocks(uint32_t n, int lanes) { return ((n - 1) / (uint32_t)lanes + 1 + 3) / 4; }
+
+// Whether a pass of first trials may run at all for a batch of n queries on a
+// grid of `blocks` blocks (trial_plan decides by the list's length).
+inline bool trial_split_possible(uint32_t n, int cap, int blocks) {
+    return (unsigned long long)n * (unsigned)cap > (unsigned long long)kTrialSinglePass * 128u * (unsigned)blocks;
+}
+
+inline uint32_t finish_blocks(uint32_t n, int num_sms) {
+    const uint32_t b = (n - 1) / 128 + 1, most = 8 * (uint32_t)num_sms;
+    return b < most ? b : most;
+}
+
+}  // namespace sms
