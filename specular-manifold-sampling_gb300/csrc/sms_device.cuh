@@ -97,6 +97,19 @@ SMS_HD f3 cross(f3 a, f3 b) {
 }
 SMS_HD float length(f3 a) { return sqrtf(dot(a, a)); }
 SMS_HD f3 normalize(f3 a) { return a * (1.f / sqrtf(dot(a, a))); }
+// Squared lengths whose rounding is pinned: which of the first two products
+// the compiler folds into a fused multiply-add otherwise depends on the code
+// around, and the Newton walks on wavy casters carry a last-bit difference into
+// another solution.
+#ifdef __CUDA_ARCH__
+SMS_HD float norm2_x(f3 a) { return __fmaf_rn(a.z, a.z, __fmaf_rn(a.x, a.x, __fmul_rn(a.y, a.y))); }
+SMS_HD float norm2_y(f3 a) { return __fmaf_rn(a.z, a.z, __fmaf_rn(a.y, a.y, __fmul_rn(a.x, a.x))); }
+#else
+SMS_HD float norm2_x(f3 a) { return dot(a, a); }
+SMS_HD float norm2_y(f3 a) { return dot(a, a); }
+#endif
+SMS_HD f3 normalize_x(f3 a) { return a * (1.f / sqrtf(norm2_x(a))); }
+SMS_HD f3 normalize_y(f3 a) { return a * (1.f / sqrtf(norm2_y(a))); }
 SMS_HD float safe_sqrt(float v) { return sqrtf(fmaxf(v, 0.f)); }
 SMS_HD float clamp1(float v) { return fminf(1.f, fmaxf(-1.f, v)); }
 

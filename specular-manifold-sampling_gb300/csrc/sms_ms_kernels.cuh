@@ -34,6 +34,14 @@
 namespace sms {
 
 constexpr unsigned kFull = 0xffffffffu;
+// Ended lanes of a warp before chain_run hands out new walks: 20,011 slab
+// points, unbiased, at 4 / 8 / 16 / 32 (a round of walks at a time) 3.42 / 3.47
+// / 3.55 / 4.05 ms.
+constexpr int kChainRefill = 4;
+// Blocks per SM of the trial kernel: what 168 registers (chains of two) let
+// reside.  More blocks with fewer registers lose to spills: 20,011 slab points
+// at 3 / 4 / 5 / 6 / 8 blocks 4.1 / 4.5 / 5.0 / 5.4 / 6.2 ms.
+constexpr int kMsWalkBlocks = 3;
 
 SMS_D M2 mmul(M2 a, M2 b) { return {a.a * b.a + a.b * b.c, a.a * b.b + a.b * b.d, a.c * b.a + a.d * b.c, a.c * b.b + a.d * b.d}; }
 SMS_D M2 msub(M2 a, M2 b) { return {a.a - b.a, a.b - b.b, a.c - b.c, a.d - b.d}; }
@@ -79,10 +87,9 @@ struct ChainOffsets {
 // keeps the direction at every hit (the MNEE seed path, :378-397).  kRough:
 // scattering about the offset normals of co (:380-382, :894-897).
 template <int K, bool kNM = false, bool kRough = false>
-SMS_D bool trace_chain(const DevScene &sc, f3 x0, f3 x1, const int *tmpl, bool check_flags, Chain<K> &c,
-                       int *shapes, uint32_t &err, LaneStats &st, bool straight = false,
-                       ChainOffsets<K> co = ChainOffsets<K>()) {
-    f3 wo = normalize(x1 - x0);
+SMS_D bool trace_chain_along(const DevScene &sc, f3 x0, f3 wo, const int *tmpl, bool check_flags, Chain<K> &c,
+                             int *shapes, uint32_t &err, LaneStats &st, bool straight = false,
+                             ChainOffsets<K> co = ChainOffsets<K>()) {
     f3 o = x0;
     float mint = kRayEps;
     if (kRough && co.draw) *co.pdf = 1.f;
@@ -130,6 +137,14 @@ SMS_D bool trace_chain(const DevScene &sc, f3 x0, f3 x1, const int *tmpl, bool c
     return true;
 }
 
+template <int K, bool kNM = false, bool kRough = false>
+SMS_D bool trace_chain(const DevScene &sc, f3 x0, f3 x1, const int *tmpl, bool check_flags, Chain<K> &c,
+                       int *shapes, uint32_t &err, LaneStats &st, bool straight = false,
+                       ChainOffsets<K> co = ChainOffsets<K>()) {
+    return trace_chain_along<K, kNM, kRough>(sc, x0, normalize(x1 - x0), tmpl, check_flags, c, shapes, err, st,
+                                             straight, co);
+}
+
 // The seed path of a walk (sample_seed_path :280-408): toward the sampled
 // point x1, or with cfg.mnee_init along the straight line toward the MNEE
 // target without scattering.
@@ -153,13 +168,13 @@ SMS_D bool vertex_anglediff(f3 xp, const Vtx &vc, f3 xn, const Vtx *vp, const Vt
     next = prev;
     c0 = c1 = 0.f;
     f3 wo = xn - vc.p;
-    float ilo = length(wo);
+    float ilo = sqrtf(norm2_x(wo));
     if (ilo < 1e-3f) return false;
     ilo = 1.f / ilo; wo = wo * ilo;
     f3 dwo_du = (vc.dp_du - wo * dot(wo, vc.dp_du)) * -ilo;
     f3 dwo_dv = (vc.dp_dv - wo * dot(wo, vc.dp_dv)) * -ilo;
     f3 wi = xp - vc.p;
-    float ili = length(wi);
+    float ili = sqrtf(norm2_x(wi));
     if (ili < 1e-3f) return false;
     ili = 1.f / ili; wi = wi * ili;
     f3 dwi_du = (vc.dp_du - wi * dot(wi, vc.dp_du)) * -ili;
@@ -382,6 +397,101 @@ SMS_D bool chain_newton(const DevScene &sc, const SolverCfg &cfg, f3 x0, f3 lp, 
         if ((c.v[i].eta == 1.f) ? refraction : !refraction) return false;
     }
     return true;
+}
+
+// Admissibility of a converged chain: every vertex reflects or refracts as its
+// ior says (newton_solver :476-497).
+template <int K>
+SMS_D bool chain_admissible(f3 x0, f3 lp, const Chain<K> &c) {
+    #pragma unroll
+    for (int i = 0; i < K; ++i) {
+        f3 xp = i == 0 ? x0 : c.v[i - 1].p, xn = i == K - 1 ? lp : c.v[i + 1].p;
+        f3 wi = normalize(xp - c.v[i].p), wo = normalize(xn - c.v[i].p);
+        bool refraction = dot(c.v[i].gn, wi) * dot(c.v[i].gn, wo) < 0.f;
+        if ((c.v[i].eta == 1.f) ? refraction : !refraction) return false;
+    }
+    return true;
+}
+
+// One lane's walk in chain_run: its seed path and Newton iterations, each one
+// chain trace and, where that completes, one step.
+template <int K>
+struct ChainWalk {
+    Chain<K> c;          // the last complete chain
+    f3 x0, lp, target;   // shading point, light point, where the next trace aims
+    f3 vp, step;         // first vertex of the last accepted chain, full Newton step from it
+    f3 offs[K];          // offset normals (rough chains)
+    int tmpl[K];         // shapes the chain has to follow
+    float beta;
+    int it;
+    bool seed;           // the next trace is the seed path
+    bool ok;             // ended: converged admissibly at c
+};
+
+// Walks of a warp, one per lane, in lockstep by chain trace: a lane whose walk
+// has ended takes the next one instead of waiting for the warp's longest (the
+// slab's walks take 16 of 30 iterations on average, but the longest of 32
+// nearly always 30).  start(want, rank, w) fills w with the walk of the lanes
+// of rank < want and says whether there was one; finish(ended, w) is called by
+// the whole warp for the lanes that ended.  Both run once kChainRefill lanes
+// have ended.  seed_chain / chain_newton above are the same walk in one piece.
+template <int K, bool kNM, bool kRough, class Start, class Finish>
+SMS_D void chain_run(const DevScene &sc, const SolverCfg &cfg, int lanes, uint32_t &err, LaneStats &st, Start start,
+                     Finish finish) {
+    const int lane = (int)(threadIdx.x & 31);
+    ChainWalk<K> w;
+    bool active = false, ended = false;
+    bool source = true;
+    while (true) {
+        const unsigned run = __ballot_sync(kFull, active);
+        const unsigned idle = ~run & (lanes == 32 ? kFull : (1u << lanes) - 1u);
+        const unsigned em = __ballot_sync(kFull, ended);
+        if (__popc(idle) >= (source ? min(kChainRefill, lanes) : 33) || run == 0u) {
+            if (em) finish(ended, w);
+            ended = false;
+            if (source) {
+                const int want = __popc(idle);
+                const bool mine = (idle >> lane) & 1u;
+                active = start(want, mine ? __popc(idle & ((1u << lane) - 1u)) : 32, w) || active;
+                if (__popc(__ballot_sync(kFull, active)) < __popc(run) + want) source = false;
+            }
+            if (__ballot_sync(kFull, active) == 0u) break;
+        }
+        if (active) {
+            ChainOffsets<K> co;
+            if constexpr (kRough) co.offs = w.offs;
+            const f3 to = w.target - w.x0;
+            const f3 wo = w.seed ? normalize_y(to) : normalize_x(to);
+            const bool hit = trace_chain_along<K, kNM, kRough>(sc, w.x0, wo, w.tmpl, w.seed, w.c, nullptr, err, st,
+                                                               w.seed && cfg.mnee_init, co);
+            bool go = true;
+            if (hit) {
+                if (!w.seed) w.beta = fminf(1.f, 2.f * w.beta);
+                w.seed = false;
+                bool conv = false;
+                float du = 0.f, dv = 0.f;
+                go = w.it < cfg.max_iterations &&
+                     chain_step<K, kRough>(cfg, w.x0, w.lp, w.c, conv, du, dv, kRough ? w.offs : nullptr);
+                if (go && conv) {
+                    w.ok = chain_admissible<K>(w.x0, w.lp, w.c);
+                    go = false;
+                }
+                w.vp = w.c.v[0].p;
+                w.step = w.c.v[0].dp_du * du + w.c.v[0].dp_dv * dv;
+            } else {
+                go = !w.seed;
+                w.beta = 0.5f * w.beta;
+            }
+            // the last iteration's chain, from which no step would be taken, is counted, not traced
+            if (go && ++w.it >= cfg.max_iterations) go = false;
+            if (go) {
+                w.target = w.vp - w.step * (cfg.step_scale * w.beta);
+            } else {
+                active = false;
+                ended = true;
+            }
+        }
+    }
 }
 
 // specular_reflectance (:920-1023): Fresnel along the re-traced chain, then
@@ -878,19 +988,14 @@ __global__ void __launch_bounds__(128) ms_first_kernel(DevScene sc, SolverCfg cf
     flush_stats(st, ctr, err, kPhaseMs);
 }
 
-// Blocks per SM of the trial kernel: what 168 registers (chains of two) let
-// reside.  More blocks with fewer registers lose to spills: 20,011 slab points
-// at 3 / 4 / 5 / 6 / 8 blocks 4.1 / 4.5 / 5.0 / 5.4 / 6.2 ms.
-constexpr int kMsWalkBlocks = 3;
-
 // Part 2: Bernoulli trials (:111-135), one lane per trial, drawn from the
 // stream of sms_trials.cuh; trial walks must reproduce the template's shapes
 // (and, kRough, scatter about its offsets).
 template <int K, bool kNM, bool kRough = false>
-__global__ void __launch_bounds__(128) ms_trials_kernel(DevScene sc, SolverCfg cfg, int ci, const float *__restrict__ qs,
-                                                        uint32_t n, uint64_t seed, uint64_t stream_off,
-                                                        int *__restrict__ count, SsScratch scr,
-                                                        const int *__restrict__ tmpl_in, DevCounters *ctr, int pass) {
+__global__ void __launch_bounds__(128, kMsWalkBlocks)
+ms_trials_kernel(DevScene sc, SolverCfg cfg, int ci, const float *__restrict__ qs, uint32_t n, uint64_t seed,
+                 uint64_t stream_off, int *__restrict__ count, SsScratch scr, const int *__restrict__ tmpl_in,
+                 DevCounters *ctr, int pass) {
     const int cap = cfg.max_trials > 0 ? cfg.max_trials : kTrialHardLimit;
     TrialStream ts(*(volatile unsigned *)&ctr->trial_count, cap, pass);
     if (ts.total == 0) return;
@@ -900,46 +1005,45 @@ __global__ void __launch_bounds__(128) ms_trials_kernel(DevScene sc, SolverCfg c
     LaneStats st;
     uint32_t err = 0;
     const int caster = sc.casters_ms[ci];
-    while (true) {
-        uint32_t qi;
-        int t;
-        const bool have = ts.next(buf, scr.list, count, ctr, pass, cfg.queue_chunk, qi, t);
-        if (!__any_sync(kFull, have)) break;
-        if (have) {
-            const Query Q = load_query(qs, n, qi);
-            Pcg32 rng = query_rng(seed, query_stream(cfg, stream_off, qi), 0);
-            Light L;
-            sample_emitter(sc, sc.emitters_ms, sc.n_emitters_ms, rng, Q.x, L);
-            const uint32_t pos = scr.pos[qi];
-            int tmpl[K];
+    uint32_t qi = 0;
+    int t = 0;
+    auto start = [&](int want, int rank, ChainWalk<K> &w) {
+        if (!ts.next(buf, scr.list, count, ctr, pass, cfg.queue_chunk, want, rank, qi, t)) return false;
+        const Query Q = load_query(qs, n, qi);
+        Pcg32 rng = query_rng(seed, query_stream(cfg, stream_off, qi), 0);
+        Light L;
+        sample_emitter(sc, sc.emitters_ms, sc.n_emitters_ms, rng, Q.x, L);
+        w.x0 = Q.x;
+        w.lp = L.p;
+        #pragma unroll
+        for (int b = 0; b < K; ++b) w.tmpl[b] = tmpl_in[(size_t)b * n + qi];
+        if constexpr (kRough) {
+            const float *orow = ms_offset_rows(const_cast<int *>(tmpl_in), n);
             #pragma unroll
-            for (int b = 0; b < K; ++b) tmpl[b] = tmpl_in[(size_t)b * n + qi];
-            f3 toff[K];
-            #pragma unroll
-            for (int b = 0; b < K; ++b) toff[b] = mk(0.f, 0.f, 1.f);
-            if constexpr (kRough) {
-                const float *orow = ms_offset_rows(const_cast<int *>(tmpl_in), n);
-                #pragma unroll
-                for (int b = 0; b < K; ++b)
-                    toff[b] = mk(orow[(size_t)(3 * b) * n + qi], orow[(size_t)(3 * b + 1) * n + qi],
-                                 orow[(size_t)(3 * b + 2) * n + qi]);
-            }
-            rng.advance((uint64_t)(pos - 3u) + kRun * (uint64_t)(t - 1));
-            float sx = rng.next_f32(), sy = rng.next_f32();
-            f3 x1 = sample_position(sc, sc.shapes[caster], sx, sy);
-            Chain<K> c;
-            int it = 0;
-            ChainOffsets<K> co;
-            co.offs = toff;
-            bool succ = seed_chain<K, kNM, kRough>(sc, cfg, caster, Q.x, x1, L.p, tmpl, c, nullptr, err, st, co) &&
-                        chain_newton<K, kNM, kRough>(sc, cfg, Q.x, L.p, tmpl, c, it, err, st, kRough ? toff : nullptr);
-            if (succ) {
-                const f3 dir0 = mk(scr.dir0[qi], scr.dir0[(size_t)n + qi], scr.dir0[2 * (size_t)n + qi]);
-                succ = fabsf(dot(dir0, normalize(c.v[0].p - Q.x)) - 1.f) < cfg.uniqueness_threshold;
-            }
-            trial_end(count, ctr, qi, t, succ, it, st);
+            for (int b = 0; b < K; ++b)
+                w.offs[b] = mk(orow[(size_t)(3 * b) * n + qi], orow[(size_t)(3 * b + 1) * n + qi],
+                               orow[(size_t)(3 * b + 2) * n + qi]);
         }
-    }
+        rng.advance((uint64_t)(scr.pos[qi] - 3u) + kRun * (uint64_t)(t - 1));
+        const float sx = rng.next_f32(), sy = rng.next_f32();
+        const f3 x1 = sample_position(sc, sc.shapes[caster], sx, sy);
+        w.target = cfg.mnee_init ? mnee_target(sc.shapes[caster], L.p) : x1;
+        w.beta = 1.f;
+        w.it = 0;
+        w.seed = true;
+        w.ok = false;
+        return true;
+    };
+    auto finish = [&](bool ended, const ChainWalk<K> &w) {
+        if (!ended) return;
+        bool succ = w.ok;
+        if (succ) {
+            const f3 dir0 = mk(scr.dir0[qi], scr.dir0[(size_t)n + qi], scr.dir0[2 * (size_t)n + qi]);
+            succ = fabsf(dot(dir0, normalize(w.c.v[0].p - w.x0)) - 1.f) < cfg.uniqueness_threshold;
+        }
+        trial_end(count, ctr, qi, t, succ, w.it, st);
+    };
+    chain_run<K, kNM, kRough>(sc, cfg, ts.plan.lanes, err, st, start, finish);
     flush_stats(st, ctr, err, kPhaseMs);
 }
 

@@ -288,7 +288,8 @@ __global__ void __launch_bounds__(128, ss_walk_blocks(kVar)) ss_trials_kernel(De
     while (true) {
         uint32_t qi;
         int t;
-        const bool have = ts.next(buf, scr.list, count, ctr, pass, cfg.queue_chunk, qi, t);
+        const bool have = ts.next(buf, scr.list, count, ctr, pass, cfg.queue_chunk, ts.plan.lanes, (int)(threadIdx.x & 31),
+                                  qi, t);
         if (!__any_sync(0xffffffffu, have)) break;
         if (have) {
             const Query Q = load_query(qs, n, qi);

@@ -81,14 +81,14 @@ struct TrialStream {
         total = (unsigned long long)n * (unsigned)max(0, plan.hi - plan.lo + 1);
     }
 
-    // Up to plan.lanes trials for lanes 0 .. k-1, in stream order; returns
-    // whether this lane has one.  Called by the whole warp.  false for every
-    // lane: the pass is done.
+    // Draw up to `want` trials (at most 32), in stream order, for the lanes
+    // of rank < want; returns whether this lane got one.  Called by the whole
+    // warp.  Fewer than want: the pass has no more.
     SMS_D bool next(TrialBuffer &buf, const uint32_t *list, const int *count, DevCounters *ctr, int pass,
-                    int chunk, uint32_t &qi, int &t) {
+                    int chunk, int want, int rank, uint32_t &qi, int &t) {
         const unsigned full = 0xffffffffu;
         const int lane = (int)(threadIdx.x & 31);
-        while (ready < plan.lanes && !drained) {
+        while (ready < want && !drained) {
             if (cur >= end) {
                 // a claim is a few rounds of the warp (chunk at least), but no
                 // more than its share of the stream
@@ -127,10 +127,10 @@ struct TrialStream {
             cur += (unsigned)k;
         }
         __syncwarp();
-        const int take = min(ready, plan.lanes);
-        const bool mine = lane < take;
-        if (mine) { qi = buf.qi[lane]; t = buf.t[lane]; }
-        // what is left moves to the front (at most plan.lanes - 1 entries)
+        const int take = min(ready, want);
+        const bool mine = rank < take;
+        if (mine) { qi = buf.qi[rank]; t = buf.t[rank]; }
+        // what is left moves to the front (fewer than 32 entries)
         uint32_t q2 = 0;
         int t2 = 0;
         const bool move = take + lane < ready;
