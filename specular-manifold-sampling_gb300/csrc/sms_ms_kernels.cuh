@@ -81,19 +81,25 @@ struct ChainOffsets {
     float *pdf = nullptr;         // first path: product of the offset densities
 };
 
-// Trace a specular chain from x0 toward x1, reflecting or refracting at each
-// hit (sample_seed_path :327-397, reproject :865-917).  tmpl (K shape ids) or
+// Trace a specular chain from x0 along wo, reflecting or refracting at each hit
+// (sample_seed_path :327-397, reproject :865-917).  tmpl (K shape ids) or
 // null; check_flags restricts hits to caster_multi / bouncer shapes; straight
 // keeps the direction at every hit (the MNEE seed path, :378-397).  kRough:
 // scattering about the offset normals of co (:380-382, :894-897).
+// The loop over the vertices stays a loop: one traversal per call site instead
+// of K.  Unrolled, the walk kernels of chains of two were so long that their
+// warps waited more for instructions (11 of 32 cycles an instruction) than for
+// memory: 65,536 slab points, biased, 36.4 -> 30.8 ms; 20,011 points, unbiased,
+// 3.42 -> 3.21 ms.  The chain then lies in local memory, which costs less.
+// Unrolling the constraint loop of chain_step pays (32.5 ms as a loop).
 template <int K, bool kNM = false, bool kRough = false>
-SMS_D bool trace_chain_along(const DevScene &sc, f3 x0, f3 wo, const int *tmpl, bool check_flags, Chain<K> &c,
-                             int *shapes, uint32_t &err, LaneStats &st, bool straight = false,
-                             ChainOffsets<K> co = ChainOffsets<K>()) {
+SMS_D bool trace_chain(const DevScene &sc, f3 x0, f3 wo, const int *tmpl, bool check_flags, Chain<K> &c,
+                       int *shapes, uint32_t &err, LaneStats &st, bool straight = false,
+                       ChainOffsets<K> co = ChainOffsets<K>()) {
     f3 o = x0;
     float mint = kRayEps;
     if (kRough && co.draw) *co.pdf = 1.f;
-    #pragma unroll
+    #pragma unroll 1
     for (int b = 0; b < K; ++b) {
         Hit h;
         trace(sc, o, wo, mint, INFINITY, false, h, err);
@@ -137,14 +143,6 @@ SMS_D bool trace_chain_along(const DevScene &sc, f3 x0, f3 wo, const int *tmpl, 
     return true;
 }
 
-template <int K, bool kNM = false, bool kRough = false>
-SMS_D bool trace_chain(const DevScene &sc, f3 x0, f3 x1, const int *tmpl, bool check_flags, Chain<K> &c,
-                       int *shapes, uint32_t &err, LaneStats &st, bool straight = false,
-                       ChainOffsets<K> co = ChainOffsets<K>()) {
-    return trace_chain_along<K, kNM, kRough>(sc, x0, normalize(x1 - x0), tmpl, check_flags, c, shapes, err, st,
-                                             straight, co);
-}
-
 // The seed path of a walk (sample_seed_path :280-408): toward the sampled
 // point x1, or with cfg.mnee_init along the straight line toward the MNEE
 // target without scattering.
@@ -153,9 +151,9 @@ SMS_D bool seed_chain(const DevScene &sc, const SolverCfg &cfg, int caster, f3 x
                       Chain<K> &c, int *shapes, uint32_t &err, LaneStats &st,
                       ChainOffsets<K> co = ChainOffsets<K>()) {
     if (cfg.mnee_init)
-        return trace_chain<K, kNM, kRough>(sc, x0, mnee_target(sc.shapes[caster], lp), tmpl, true, c, shapes, err,
-                                           st, true, co);
-    return trace_chain<K, kNM, kRough>(sc, x0, x1, tmpl, true, c, shapes, err, st, false, co);
+        return trace_chain<K, kNM, kRough>(sc, x0, normalize_y(mnee_target(sc.shapes[caster], lp) - x0), tmpl, true, c,
+                                           shapes, err, st, true, co);
+    return trace_chain<K, kNM, kRough>(sc, x0, normalize_y(x1 - x0), tmpl, true, c, shapes, err, st, false, co);
 }
 
 // Angle-difference constraint of vertex i and its blocks w.r.t. the previous,
@@ -378,7 +376,7 @@ SMS_D bool chain_newton(const DevScene &sc, const SolverCfg &cfg, f3 x0, f3 lp, 
         if (it + 1 >= cfg.max_iterations) { it++; break; }
         f3 p0 = c.v[0].p - (c.v[0].dp_du * du + c.v[0].dp_dv * dv) * (cfg.step_scale * beta);
         Chain<K> prop;
-        if (trace_chain<K, kNM, kRough>(sc, x0, p0, tmpl, false, prop, nullptr, err, st, false, co)) {
+        if (trace_chain<K, kNM, kRough>(sc, x0, normalize_x(p0 - x0), tmpl, false, prop, nullptr, err, st, false, co)) {
             beta = fminf(1.f, 2.f * beta);
             c = prop;
             need = true;
@@ -462,8 +460,8 @@ SMS_D void chain_run(const DevScene &sc, const SolverCfg &cfg, int lanes, uint32
             if constexpr (kRough) co.offs = w.offs;
             const f3 to = w.target - w.x0;
             const f3 wo = w.seed ? normalize_y(to) : normalize_x(to);
-            const bool hit = trace_chain_along<K, kNM, kRough>(sc, w.x0, wo, w.tmpl, w.seed, w.c, nullptr, err, st,
-                                                               w.seed && cfg.mnee_init, co);
+            const bool hit = trace_chain<K, kNM, kRough>(sc, w.x0, wo, w.tmpl, w.seed, w.c, nullptr, err, st,
+                                                         w.seed && cfg.mnee_init, co);
             bool go = true;
             if (hit) {
                 if (!w.seed) w.beta = fminf(1.f, 2.f * w.beta);
