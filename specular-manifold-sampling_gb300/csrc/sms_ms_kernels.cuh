@@ -367,23 +367,22 @@ SMS_D bool chain_newton(const DevScene &sc, const SolverCfg &cfg, f3 x0, f3 lp, 
     it = 0;
     float beta = 1.f;
     bool need = true, conv = false, ok = true;
-    float du = 0.f, dv = 0.f;
+    // first vertex of the last complete chain and the full Newton step from it
+    f3 vp = splat(0.f), step = vp;
     while (it < cfg.max_iterations) {
-        if (need) ok = chain_step<K, kRough>(cfg, x0, lp, c, conv, du, dv, offs);
+        if (need) {
+            float du = 0.f, dv = 0.f;
+            ok = chain_step<K, kRough>(cfg, x0, lp, c, conv, du, dv, offs);
+            vp = c.v[0].p;
+            step = c.v[0].dp_du * du + c.v[0].dp_dv * dv;
+        }
         if (!ok) break;
         if (conv) break;
         // the last iteration's chain would be one no step is taken from
         if (it + 1 >= cfg.max_iterations) { it++; break; }
-        f3 p0 = c.v[0].p - (c.v[0].dp_du * du + c.v[0].dp_dv * dv) * (cfg.step_scale * beta);
-        Chain<K> prop;
-        if (trace_chain<K, kNM, kRough>(sc, x0, normalize_x(p0 - x0), tmpl, false, prop, nullptr, err, st, false, co)) {
-            beta = fminf(1.f, 2.f * beta);
-            c = prop;
-            need = true;
-        } else {
-            beta = 0.5f * beta;
-            need = false;
-        }
+        const f3 p0 = vp - step * (cfg.step_scale * beta);
+        need = trace_chain<K, kNM, kRough>(sc, x0, normalize_x(p0 - x0), tmpl, false, c, nullptr, err, st, false, co);
+        beta = need ? fminf(1.f, 2.f * beta) : 0.5f * beta;
         it++;
     }
     if (!(ok && conv)) return false;
