@@ -46,7 +46,13 @@
 namespace sms {
 namespace {
 
-constexpr int kPtBlock = 256;
+// Blocks of 128 threads, 8 an SM for the bounce kernel (64 registers): its warps
+// wait for tree nodes one after another, and more of them hide more than the
+// spills cost.  A 512 x 384 image of the pool, 16 spp, at 256 x 2 (114
+// registers) / 256 x 3 / 256 x 4 / 128 x 5 / 128 x 6 / 128 x 8 / 64 x 16:
+// 7.8 / 7.0 / 6.8 / 7.0 / 6.8 / 6.5 / 6.5 ms.
+constexpr int kPtBlock = 128;
+constexpr int kBounceBlocks = 8;
 constexpr uint32_t kPtDefaultPaths = 1u << 20;
 constexpr int kPtHardDepth = 4096;        // bounce limit of an unbounded path
 constexpr int kQueryRowsMax = 21;        // glint queries; single / multi scatter use 16
@@ -62,6 +68,8 @@ constexpr int kRecDefault = 0, kRecReceiver = 1, kRecCaster = 2, kRecEmitter = 3
 constexpr int kTfShift = 8;
 constexpr int kTfDefault = 0, kTfReceiver = 1, kTfSingleCaster = 2, kTfSingleEmitter = 3, kTfMultiCaster = 4,
               kTfMultiEmitter = 5;
+// what a slot of a bounce leaves behind
+constexpr int kWantQuery = 1, kWantLive = 2;
 // rows of the MNEE record: receiver point (3), first specular shape (int
 // bits), specular vertices (3 per bounce)
 constexpr int kMneeRows = 4 + 3 * kMaxBounces;
@@ -99,15 +107,16 @@ struct PtState {
     int *hit_shape, *flags;               // cap
     uint32_t *hit_prim;                   // cap
     float *stage;                         // kStageRows x cap
-    int *want;                            // cap
+    int *want;                            // cap, per slot of the bounce: kWantQuery | kWantLive
     // path_sms_ms unbiased MNEE (MNEEHelper, path_sms_ms.cpp:54-142): per
     // path the receiver point, the first specular shape and the specular
     // vertices since (kMneeRows x cap; null when off), and the paths whose
     // emitter hit awaits the MNEE test of this bounce
     float *mnee;
     int *mnee_want;
-    uint32_t *block_q, *block_a;          // per block
+    uint64_t *block_n;                    // per block: queries (high half), live paths; then their offsets
     uint32_t *totals;                     // [0] queries, [1] live paths
+    uint32_t *live[2];                    // cap each: the paths of a bounce, in path order (odd / even bounces)
     // pending SMS batch (qcap entries, appended bounce by bounce)
     int qrows;                            // query rows: 16, or 21 for glints
     float *qraw;                          // qrows x qcap, stride qcap
@@ -574,14 +583,23 @@ SMS_D float cam_importance(const PtCam &cam, f3 d) {
 }
 
 // ------------------------------------------------------------------ bounce
+// The path of a slot of a bounce: the first bounce has a slot per path, later
+// ones a slot per path alive, listed by pt_gather_kernel.  A slot per path in
+// every bounce left 8, 4, 2 of 32 lanes a path to follow from the second bounce
+// on (a 512 x 384 image of the pool, 16 spp: 10.9 -> 7.8 ms).
+SMS_D uint32_t bounce_path(const PtState &S, int depth, uint32_t slot, uint32_t n) {
+    return depth > 1 && slot < n ? S.live[depth & 1][slot] : slot;
+}
+
 template <bool kMneeCheck>
-__global__ void __launch_bounds__(kPtBlock) pt_bounce_kernel(DevScene sc, PtParams P, PtState S, int depth,
+__global__ void __launch_bounds__(kPtBlock, kBounceBlocks) pt_bounce_kernel(DevScene sc, PtParams P, PtState S, int depth,
                                                              uint32_t n, DevCounters *ctr, PtCam cam) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t i = bounce_path(S, depth, slot, n);
     int want = 0, alive_out = 0;
     uint32_t err = 0;
-    if (i < n && S.mnee_want) S.mnee_want[i] = 0;
-    if (i < n && (S.flags[i] & kAlive)) {
+    if (slot < n && S.mnee_want) S.mnee_want[i] = 0;
+    if (slot < n && (S.flags[i] & kAlive)) {
         int flags = S.flags[i];
         Pcg32 rng = load_rng(S, i);
         f3 o = ld3s(S.o, S.cap, i), d = ld3s(S.d, S.cap, i);
@@ -979,83 +997,80 @@ __global__ void __launch_bounds__(kPtBlock) pt_bounce_kernel(DevScene sc, PtPara
         store_rng(S, i, rng);
         alive_out = alive;
     }
-    if (i < n) S.want[i] = want;
+    if (slot < n) S.want[slot] = (want ? kWantQuery : 0) | (alive_out ? kWantLive : 0);
     const int bq = __syncthreads_count(want);
     const int ba = __syncthreads_count(alive_out);
-    if (threadIdx.x == 0) {
-        S.block_q[blockIdx.x] = (uint32_t)bq;
-        S.block_a[blockIdx.x] = (uint32_t)ba;
-    }
+    if (threadIdx.x == 0) S.block_n[blockIdx.x] = ((uint64_t)bq << 32) | (uint32_t)ba;
     if (err) atomicOr(&ctr->error, err);
 }
 
 // ------------------------------------------------------------ compaction
-// Exclusive prefix sum of the per-block query counts (one block, in order)
-// and the totals of queries and live paths.
+// Exclusive prefix sum of the per-block counts of queries and live paths (one
+// block, in order) and their totals.
 __global__ void __launch_bounds__(1024) pt_scan_kernel(PtState S, uint32_t n_blocks) {
-    __shared__ uint32_t warp_sum[32];
-    __shared__ uint32_t carry;
-    __shared__ uint32_t alive_sum;
-    if (threadIdx.x == 0) { carry = 0; alive_sum = 0; }
+    __shared__ uint64_t warp_sum[32];
+    __shared__ uint64_t carry;
+    if (threadIdx.x == 0) carry = 0;
     __syncthreads();
     const unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    uint32_t alive_local = 0;
-    for (uint32_t b0 = 0; b0 < n_blocks; b0 += 1024) {
-        const uint32_t b = b0 + threadIdx.x;
-        const uint32_t v = b < n_blocks ? S.block_q[b] : 0u;
-        alive_local += b < n_blocks ? S.block_a[b] : 0u;
-        uint32_t x = v;
+    auto inclusive = [&](uint64_t x) {
         #pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
-            uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
+            const uint64_t y = __shfl_up_sync(0xffffffffu, x, off);
             if ((int)lane >= off) x += y;
         }
+        return x;
+    };
+    for (uint32_t b0 = 0; b0 < n_blocks; b0 += 1024) {
+        const uint32_t b = b0 + threadIdx.x;
+        const uint64_t v = b < n_blocks ? S.block_n[b] : 0u;
+        const uint64_t x = inclusive(v);
         if (lane == 31) warp_sum[wid] = x;
         __syncthreads();
-        if (wid == 0) {
-            uint32_t w = warp_sum[lane];
-            #pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                uint32_t y = __shfl_up_sync(0xffffffffu, w, off);
-                if ((int)lane >= off) w += y;
-            }
-            warp_sum[lane] = w;   // inclusive
-        }
+        if (wid == 0) warp_sum[lane] = inclusive(warp_sum[lane]);
         __syncthreads();
-        const uint32_t before = carry + (wid ? warp_sum[wid - 1] : 0u) + x - v;
-        if (b < n_blocks) S.block_q[b] = before;   // now the block's offset
+        if (b < n_blocks) S.block_n[b] = carry + (wid ? warp_sum[wid - 1] : 0u) + x - v;   // now the block's offsets
         __syncthreads();
         if (threadIdx.x == 0) carry += warp_sum[31];
         __syncthreads();
     }
-    atomicAdd(&alive_sum, alive_local);
-    __syncthreads();
     if (threadIdx.x == 0) {
-        S.totals[0] = carry;
-        S.totals[1] = alive_sum;
+        S.totals[0] = (uint32_t)(carry >> 32);
+        S.totals[1] = (uint32_t)carry;
     }
 }
 
-// Staged queries of this bounce -> entries base + r of the pending batch
-// (r = rank in path order); their stream is path + bounce * 2^48.
+// The slots of a bounce: staged queries -> entries base + r of the pending
+// batch (r = rank in path order), their stream path + bounce * 2^48; live
+// paths -> the next bounce's list, in path order.
 __global__ void __launch_bounds__(kPtBlock) pt_gather_kernel(PtState S, uint32_t n, uint32_t base, uint64_t g0,
                                                              int depth) {
-    __shared__ uint32_t warp_cnt[kPtBlock / 32];
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int w = i < n ? S.want[i] : 0;
-    const unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const unsigned m = __ballot_sync(0xffffffffu, w);
-    if (lane == 0) warp_cnt[wid] = __popc(m);
+    __shared__ uint32_t warp_q[kPtBlock / 32], warp_a[kPtBlock / 32];
+    const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t i = bounce_path(S, depth, slot, n);
+    const int w = slot < n ? S.want[slot] : 0;
+    const unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5, below = (1u << lane) - 1u;
+    const unsigned mq = __ballot_sync(0xffffffffu, w & kWantQuery), ma = __ballot_sync(0xffffffffu, w & kWantLive);
+    if (lane == 0) { warp_q[wid] = __popc(mq); warp_a[wid] = __popc(ma); }
     __syncthreads();
-    if (!w) return;
-    uint32_t r = S.block_q[blockIdx.x] + __popc(m & ((1u << lane) - 1u));
-    for (unsigned k = 0; k < wid; ++k) r += warp_cnt[k];
-    const uint32_t e = base + r;
-    for (int k = 0; k < S.qrows; ++k) S.qraw[(size_t)k * S.qcap + e] = S.stage[(size_t)k * S.cap + i];
-    #pragma unroll
-    for (int k = 0; k < 3; ++k) S.qw[(size_t)k * S.qcap + e] = S.stage[(size_t)(21 + k) * S.cap + i];
-    S.qmap[e] = i;
-    S.qstream[e] = g0 + i + ((uint64_t)depth << 48);
+    const uint64_t off = S.block_n[blockIdx.x];
+    // the MNEE test of this bounce is done; a path that ends here is not visited again
+    if (slot < n && S.mnee_want) S.mnee_want[i] = 0;
+    if (w & kWantLive) {
+        uint32_t r = (uint32_t)off + __popc(ma & below);
+        for (unsigned k = 0; k < wid; ++k) r += warp_a[k];
+        S.live[(depth + 1) & 1][r] = i;
+    }
+    if (w & kWantQuery) {
+        uint32_t r = (uint32_t)(off >> 32) + __popc(mq & below);
+        for (unsigned k = 0; k < wid; ++k) r += warp_q[k];
+        const uint32_t e = base + r;
+        for (int k = 0; k < S.qrows; ++k) S.qraw[(size_t)k * S.qcap + e] = S.stage[(size_t)k * S.cap + i];
+        #pragma unroll
+        for (int k = 0; k < 3; ++k) S.qw[(size_t)k * S.qcap + e] = S.stage[(size_t)(21 + k) * S.cap + i];
+        S.qmap[e] = i;
+        S.qstream[e] = g0 + i + ((uint64_t)depth << 48);
+    }
 }
 
 // Pending batch (stride qcap) -> packed SoA queries (stride nq).
@@ -1376,7 +1391,7 @@ extern "C" sms_status sms_render_device(sms_ctx *c, const sms_camera *cam, const
                  o_hu = take(4 * (size_t)cap), o_hv = take(4 * (size_t)cap), o_hs = take(4 * (size_t)cap),
                  o_fl = take(4 * (size_t)cap), o_hp = take(4 * (size_t)cap), o_cs = take(8 * (size_t)cap),
                  o_st = take(4 * (size_t)kStageRows * cap), o_w = take(4 * (size_t)cap),
-                 o_bq = take(4 * (size_t)n_blocks_cap), o_ba = take(4 * (size_t)n_blocks_cap), o_tot = take(16),
+                 o_bn = take(8 * (size_t)n_blocks_cap), o_tot = take(16), o_lv = take(8 * (size_t)cap),
                  o_qr = take(4 * (size_t)kQueryRowsMax * qcap), o_qw = take(12 * (size_t)qcap),
                  o_qm = take(4 * (size_t)qcap), o_qs = take(8 * (size_t)qcap),
                  o_q = take(4 * (size_t)kQueryRowsMax * qcap), o_val = take(12 * (size_t)qcap),
@@ -1451,8 +1466,9 @@ extern "C" sms_status sms_render_device(sms_ctx *c, const sms_camera *cam, const
     S.cam_s = reinterpret_cast<float *>(blk + o_cs);
     S.stage = reinterpret_cast<float *>(blk + o_st);
     S.want = reinterpret_cast<int *>(blk + o_w);
-    S.block_q = reinterpret_cast<uint32_t *>(blk + o_bq);
-    S.block_a = reinterpret_cast<uint32_t *>(blk + o_ba);
+    S.block_n = reinterpret_cast<uint64_t *>(blk + o_bn);
+    S.live[0] = reinterpret_cast<uint32_t *>(blk + o_lv);
+    S.live[1] = S.live[0] + cap;
     S.totals = reinterpret_cast<uint32_t *>(blk + o_tot);
     S.qraw = reinterpret_cast<float *>(blk + o_qr);
     S.qw = reinterpret_cast<float *>(blk + o_qw);
@@ -1491,29 +1507,30 @@ extern "C" sms_status sms_render_device(sms_ctx *c, const sms_camera *cam, const
         const uint32_t nb = (n + kPtBlock - 1) / kPtBlock;
         pt_camera_kernel<<<nb, kPtBlock, 0, s>>>(*v.scene, pc, S, g0, n, P.seed, teaser ? (tp == 0 ? 1 : 0) : 1);
         PT_TRY(cudaGetLastError());
-        uint32_t alive_bound = n;   // paths that can stage a query at the next bounce
+        uint32_t live = n;   // slots of the next bounce: all paths, then those alive
         for (int depth = 1;; ++depth) {
             if (depth > kPtHardDepth) {
                 st = rfail(SMS_ERR_DEVICE_LIMIT, "sms_render: a path exceeded 4096 bounces (raise rr pressure or "
                                                  "bound max_depth)");
                 goto done;
             }
-            if (pending + alive_bound > qcap) {
+            if (pending + live > qcap) {
                 st = flush();
                 if (st) goto done;
             }
+            const uint32_t lb = (live + kPtBlock - 1) / kPtBlock;
             if (P.mnee_check)
-                pt_bounce_kernel<true><<<nb, kPtBlock, 0, s>>>(*v.scene, P, S, depth, n, v.counters, pc);
+                pt_bounce_kernel<true><<<lb, kPtBlock, 0, s>>>(*v.scene, P, S, depth, live, v.counters, pc);
             else
-                pt_bounce_kernel<false><<<nb, kPtBlock, 0, s>>>(*v.scene, P, S, depth, n, v.counters, pc);
+                pt_bounce_kernel<false><<<lb, kPtBlock, 0, s>>>(*v.scene, P, S, depth, live, v.counters, pc);
             PT_TRY(cudaGetLastError());
             if (P.mnee_ms) {
                 PT_TRY(launch_ms_mnee_check(*v.scene, P.solver, P.bounces, S.mnee, S.stage, S.mnee_want, S.L, n,
                                             S.cap, v.counters, s));
             }
-            pt_scan_kernel<<<1, 1024, 0, s>>>(S, nb);
+            pt_scan_kernel<<<1, 1024, 0, s>>>(S, lb);
             PT_TRY(cudaGetLastError());
-            pt_gather_kernel<<<nb, kPtBlock, 0, s>>>(S, n, pending, g0, depth);
+            pt_gather_kernel<<<lb, kPtBlock, 0, s>>>(S, live, pending, g0, depth);
             PT_TRY(cudaGetLastError());
             PT_TRY(cudaMemcpyAsync(host_tot, S.totals, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
             PT_TRY(cudaStreamSynchronize(s));
@@ -1523,8 +1540,8 @@ extern "C" sms_status sms_render_device(sms_ctx *c, const sms_camera *cam, const
                 seg_cnt.push_back(nq);
                 pending += nq;
             }
-            alive_bound = n_alive;
-            if (n_alive == 0) break;
+            live = n_alive;
+            if (live == 0) break;
         }
         st = flush();
         if (st) goto done;
