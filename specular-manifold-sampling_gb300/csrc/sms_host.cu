@@ -10,6 +10,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -511,6 +512,8 @@ struct sms_ctx {
     // estimator only: rough multi-scatter chain shapes / glinty shapes
     bool ms_rough = false, glint_rough = false;
     bool ms_nm = false;   // a multi-scatter chain shape carries the normal map
+    std::mutex render_mutex;   // guards render_buf
+    RenderBuffers render_buf;  // of the last render, kept for the next (ctx_give_render)
     uint32_t render_spp = 0;   // samples per pixel of the last render
     bool nm_rough = false;   // the normal-mapped shape is rough
     float *lean = nullptr;   // LEAN pyramid of the slope map (glints integrator), built on first use
@@ -559,6 +562,8 @@ extern "C" void sms_ctx_destroy(sms_ctx *c) {
     if (c->io) cudaFree(c->io);
     if (c->scratch) cudaFree(c->scratch);
     if (c->lean) cudaFree(c->lean);
+    if (c->render_buf.block) cudaFree(c->render_buf.block);
+    if (c->render_buf.host) cudaFreeHost(c->render_buf.host);
     if (c->ms_tmpl) cudaFree(c->ms_tmpl);
     if (c->gmm) cudaFree(c->gmm);
     for (sms_proposal *p : c->proposals) proposal_detach(p);
@@ -1305,6 +1310,45 @@ sms_status ctx_glint_connect(sms_ctx *c, const float *q, uint32_t n, uint64_t se
 extern "C" sms_status sms_glint_connect_batch_device(sms_ctx *c, const float *q, uint32_t n, uint64_t seed,
                                                      uint64_t stream_off, sms_result *out) {
     return ctx_glint_connect(c, q, n, seed, stream_off, nullptr, out);
+}
+
+// A render's path state (643 MB for the default wavefront with SMS queries) and
+// its pinned words took 0.8 ms to allocate and free, as long as a small image
+// takes to render.
+constexpr size_t kRenderKeepBytes = (size_t)1 << 30;
+
+cudaError_t ctx_take_render(sms_ctx *c, size_t bytes, RenderBuffers &out) {
+    {
+        std::lock_guard<std::mutex> lock(c->render_mutex);
+        out = c->render_buf;
+        c->render_buf = RenderBuffers{};
+    }
+    cudaError_t e = cudaSuccess;
+    if (out.bytes < bytes) {
+        if (out.block) cudaFree(out.block);
+        out.block = nullptr;
+        out.bytes = 0;
+        e = cudaMalloc(&out.block, bytes);
+        if (e == cudaSuccess) out.bytes = bytes;
+    }
+    if (e == cudaSuccess && !out.host) e = cudaMallocHost(&out.host, 2 * sizeof(uint32_t));
+    return e;
+}
+
+void ctx_give_render(sms_ctx *c, RenderBuffers &buf) {
+    if (buf.bytes > kRenderKeepBytes) {
+        cudaFree(buf.block);
+        buf.block = nullptr;
+        buf.bytes = 0;
+    }
+    {
+        // the larger block stays
+        std::lock_guard<std::mutex> lock(c->render_mutex);
+        if (buf.bytes >= c->render_buf.bytes) std::swap(buf, c->render_buf);
+    }
+    if (buf.block) cudaFree(buf.block);
+    if (buf.host) cudaFreeHost(buf.host);
+    buf = RenderBuffers{};
 }
 
 void ctx_set_render_spp(sms_ctx *c, uint32_t spp) {

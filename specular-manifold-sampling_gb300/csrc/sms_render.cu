@@ -1290,9 +1290,8 @@ static bool camera_params(const sms_camera *c, PtCam &out, std::string &why) {
     return true;
 }
 
-extern "C" sms_status sms_render_device(sms_ctx *c, const sms_camera *cam, const sms_render_options *opt,
-                                        float *image) {
-    if (!c || !cam || !opt || !image) return rfail(SMS_ERR_INVALID_ARG, "sms_render_device: null argument");
+// The image goes to `image` (device memory) or, if that is null, to `host`.
+static sms_status render(sms_ctx *c, const sms_camera *cam, const sms_render_options *opt, float *image, float *host) {
     CtxView v;
     if (!ctx_view(c, v)) return rfail(SMS_ERR_INVALID_ARG, "sms_render_device: bad context");
     PtCam pc;
@@ -1391,7 +1390,7 @@ extern "C" sms_status sms_render_device(sms_ctx *c, const sms_camera *cam, const
     uint32_t cap = opt->max_paths ? opt->max_paths : kPtDefaultPaths;
     if (wh <= cap) cap = (uint32_t)(std::min<uint64_t>(cap / wh, (uint64_t)opt->spp) * wh);
     cap = std::max<uint32_t>(cap, 1u);
-    const uint32_t qcap = 2u * cap;
+    const uint32_t qcap = queries ? 2u * cap : 0u;
     const uint32_t n_blocks_cap = (cap + kPtBlock - 1) / kPtBlock;
 
     // one device block for the whole path state and the pending SMS batch
@@ -1402,14 +1401,16 @@ extern "C" sms_status sms_render_device(sms_ctx *c, const sms_camera *cam, const
                  o_pp = take(12 * (size_t)cap), o_eta = take(4 * (size_t)cap), o_ht = take(4 * (size_t)cap),
                  o_hu = take(4 * (size_t)cap), o_hv = take(4 * (size_t)cap), o_hs = take(4 * (size_t)cap),
                  o_fl = take(4 * (size_t)cap), o_hp = take(4 * (size_t)cap), o_cs = take(8 * (size_t)cap),
-                 o_st = take(4 * (size_t)kStageRows * cap), o_w = take(4 * (size_t)cap),
+                 o_st = take(queries ? 4 * (size_t)kStageRows * cap : 0), o_w = take(4 * (size_t)cap),
                  o_bn = take(8 * (size_t)n_blocks_cap), o_tot = take(16), o_lv = take(8 * (size_t)cap),
                  o_qr = take(4 * (size_t)kQueryRowsMax * qcap), o_qw = take(12 * (size_t)qcap),
                  o_qm = take(4 * (size_t)qcap), o_qs = take(8 * (size_t)qcap),
                  o_q = take(4 * (size_t)kQueryRowsMax * qcap), o_val = take(12 * (size_t)qcap),
                  o_cnt = take(4 * (size_t)qcap), o_wk = take(4 * (size_t)qcap),
                  o_mn = take(P.mnee_ms ? 4 * (size_t)kMneeRows * cap : 0),
-                 o_mw = take(P.mnee_ms ? 4 * (size_t)cap : 0), o_ws = take(gauss ? 4 * (size_t)wh : 0);
+                 o_mw = take(P.mnee_ms ? 4 * (size_t)cap : 0), o_ws = take(gauss ? 4 * (size_t)wh : 0),
+                 o_im = take(image ? 0 : 12 * (size_t)wh);
+    RenderBuffers buf;
     char *blk = nullptr;
     float *wsum = nullptr;   // the Gaussian filter's weight per pixel
     uint32_t *host_tot = nullptr;
@@ -1459,8 +1460,10 @@ extern "C" sms_status sms_render_device(sms_ctx *c, const sms_camera *cam, const
         return SMS_OK;
     };
     PT_TRY(cudaSetDevice(v.device));
-    PT_TRY(cudaMalloc(&blk, bytes));
-    PT_TRY(cudaMallocHost(&host_tot, 2 * sizeof(uint32_t)));
+    PT_TRY(ctx_take_render(c, bytes, buf));
+    blk = buf.block;
+    host_tot = buf.host;
+    if (!image) image = reinterpret_cast<float *>(blk + o_im);
     S.rng_state = reinterpret_cast<uint64_t *>(blk + o_rs);
     S.rng_inc = reinterpret_cast<uint64_t *>(blk + o_ri);
     S.o = reinterpret_cast<float *>(blk + o_o);
@@ -1526,7 +1529,7 @@ extern "C" sms_status sms_render_device(sms_ctx *c, const sms_camera *cam, const
                                                  "bound max_depth)");
                 goto done;
             }
-            if (pending + live > qcap) {
+            if (queries && pending + live > qcap) {
                 st = flush();
                 if (st) goto done;
             }
@@ -1592,31 +1595,24 @@ extern "C" sms_status sms_render_device(sms_ctx *c, const sms_camera *cam, const
         ctx_set_render_spp(c, spp_done);
     }
     st = ctx_check_device_error(c);
-done:
-    if (blk) {
-        cudaStreamSynchronize(s);
-        cudaFree(blk);
+    if (st == SMS_OK && host) {
+        PT_TRY(cudaMemcpyAsync(host, image, img_n * sizeof(float), cudaMemcpyDeviceToHost, s));
+        PT_TRY(cudaStreamSynchronize(s));
     }
-    if (host_tot) cudaFreeHost(host_tot);
+done:
+    if (st != SMS_OK) cudaStreamSynchronize(s);
+    ctx_give_render(c, buf);
     return st;
+}
+
+extern "C" sms_status sms_render_device(sms_ctx *c, const sms_camera *cam, const sms_render_options *opt,
+                                        float *image) {
+    if (!c || !cam || !opt || !image) return rfail(SMS_ERR_INVALID_ARG, "sms_render_device: null argument");
+    return render(c, cam, opt, image, nullptr);
 }
 
 extern "C" sms_status sms_render(sms_ctx *c, const sms_camera *cam, const sms_render_options *opt, float *image) {
     if (!c || !cam || !opt || !image) return rfail(SMS_ERR_INVALID_ARG, "sms_render: null argument");
     if (cam->width <= 0 || cam->height <= 0) return rfail(SMS_ERR_INVALID_ARG, "sms_render: bad film size");
-    CtxView v;
-    if (!ctx_view(c, v)) return rfail(SMS_ERR_INVALID_ARG, "sms_render: bad context");
-    const size_t bytes = 3 * (size_t)cam->width * (size_t)cam->height * sizeof(float);
-    float *dimg = nullptr;
-    cudaError_t e = cudaSetDevice(v.device);
-    if (e == cudaSuccess) e = cudaMalloc(&dimg, bytes);
-    if (e != cudaSuccess) return rfail(SMS_ERR_CUDA, std::string("sms_render: ") + cudaGetErrorString(e));
-    sms_status st = sms_render_device(c, cam, opt, dimg);
-    if (st == SMS_OK) {
-        e = cudaMemcpyAsync(image, dimg, bytes, cudaMemcpyDeviceToHost, v.stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(v.stream);
-        if (e != cudaSuccess) st = rfail(SMS_ERR_CUDA, std::string("sms_render: ") + cudaGetErrorString(e));
-    }
-    cudaFree(dimg);
-    return st;
+    return render(c, cam, opt, nullptr, image);
 }

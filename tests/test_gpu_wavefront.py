@@ -30,3 +30,36 @@ def test_live_paths_and_finish(sms, workloads, gpu_lib, integrator, size, max_pa
     ctx.close()
     assert np.array_equal(full, again)
     _same(full, part)
+
+
+def test_render_buffers_are_kept_and_shared(sms, workloads, gpu_lib):
+    """A context's render buffers serve images of any size and integrator in
+    any order, and two threads at a time: every image equals a new context's."""
+    import threading
+    W = workloads
+    desc, cfg = W.pool_scene(res=32), W.water_config()
+    jobs = [(7, 5, "path_sms_ss", 1), (120, 90, "path", 2), (16, 16, "path_sms_ss", 2), (50, 2, "path", 1)]
+    opt = {j: sms.RenderOptions(integrator=j[2], spp=j[3], seed=2) for j in jobs}
+    want = {}
+    for j in jobs:
+        ctx = sms.Context(sms.Scene(desc), cfg)
+        want[j] = ctx.render(W.pool_camera(*j[:2]), opt[j])
+        ctx.close()
+    ctx = sms.Context(sms.Scene(desc), cfg)
+    for j in jobs + jobs[::-1]:
+        assert np.array_equal(ctx.render(W.pool_camera(*j[:2]), opt[j]), want[j]), j
+    got = {}
+
+    def work(j):
+        got[j] = [ctx.render(W.pool_camera(*j[:2]), opt[j]) for _ in range(4)]
+
+    threads = [threading.Thread(target=work, args=(j,)) for j in jobs if j[2] == "path"]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(timeout=60)
+    ctx.close()
+    for j, images in got.items():
+        for img in images:
+            assert np.array_equal(img, want[j]), j
+    assert len(got) == 2
