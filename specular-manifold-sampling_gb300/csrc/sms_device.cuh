@@ -165,6 +165,21 @@ struct Pcg32 {
     }
 };
 
+// The map of k steps of the generator, x -> mult x + sum inc: what advance(k)
+// works out anew for every stream.
+struct PcgSkip {
+    uint64_t mult = 1u, sum = 0u;
+    SMS_HD constexpr explicit PcgSkip(uint64_t k) {
+        uint64_t m = 6364136223846793005ULL, s = 1u;
+        for (; k > 0; k >>= 1u) {
+            if (k & 1u) { sum = sum * m + s; mult *= m; }
+            s = (m + 1u) * s;
+            m *= m;
+        }
+    }
+    SMS_HD constexpr void apply(Pcg32 &r) const { r.state = mult * r.state + sum * r.inc; }
+};
+
 // --------------------------------------------------------------- scene data
 enum : int { kShapeSphere = 0, kShapeMesh = 1 };
 // shape flags (same bits as SMS_SHAPE_* in sms_gb300.h)
