@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(128) mlp_forward_kernel(MlpDev m, const float 
     __nv_bfloat16 *sw = reinterpret_cast<__nv_bfloat16 *>(smem_raw);
     float *stage = reinterpret_cast<float *>(smem_raw + (size_t)kWeightsFwd * 2) + (threadIdx.x / 32) * kStageFloats;
     stage_weights(m.wbf, sw, kWeightsFwd);
-    __syncthreads();
+    stage_wait();
     const int lane = threadIdx.x & 31;
     const uint32_t wpb = blockDim.x / 32;
     for (uint32_t w = blockIdx.x * wpb + threadIdx.x / 32; (size_t)w * 16 < n; w += gridDim.x * wpb) {
@@ -128,6 +128,11 @@ __global__ void __launch_bounds__(128) mlp_forward_kernel(MlpDev m, const float 
 }
 
 // ------------------------------------------------------------------ training
+// A serial chain per warp, one warp per scheduler and block per SM (shared
+// memory): bound by its latency, 44 us at 8,192 samples (91 -> 67 us from a cold
+// cache).  The weights come asynchronously while the inputs are encoded, both
+// halves of the warp encode, and the fragments leave transposed, two samples a
+// store.
 __global__ void __launch_bounds__(128) mlp_train_fb_kernel(MlpDev m, const float *__restrict__ feat,
                                                            const float *__restrict__ uv, size_t ld, uint32_t n_data,
                                                            int batch, int shuffle) {
@@ -137,23 +142,24 @@ __global__ void __launch_bounds__(128) mlp_train_fb_kernel(MlpDev m, const float
     float *stage = reinterpret_cast<float *>(smem_raw + (size_t)kWeightsAll * 2) + 4 * kZsFloats +
                    (threadIdx.x / 32) * kStageFloats;
     stage_weights(m.wbf, sw, kWeightsAll);
-    __syncthreads();
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int b0 = (blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32) * 16;
-    if (b0 >= batch) return;   // whole warps only (batch is a multiple of 16)
     const uint32_t step = *m.step;
     auto row_of = [&](int r) -> uint32_t {
         const uint32_t b = (uint32_t)(b0 + r);
         return shuffle ? hash32(step * 0x9E3779B9u ^ hash32(b)) % n_data : b % n_data;
     };
-    float xn[kIn];
-    {
+    __nv_bfloat16 *sx = reinterpret_cast<__nv_bfloat16 *>(stage);
+    if (b0 < batch) {
+        // while the weights come
+        float xn[kIn];
         const uint32_t r = row_of(lane & 15);
         #pragma unroll
         for (int k = 0; k < kIn; ++k) xn[k] = (__ldg(feat + (size_t)k * ld + r) - m.shift[k]) * m.scale[k];
+        stage_inputs(xn, sx);
     }
-    __nv_bfloat16 *sx = reinterpret_cast<__nv_bfloat16 *>(stage);
-    stage_inputs(xn, sx);
+    stage_wait();
+    if (b0 >= batch) return;   // whole warps only (batch is a multiple of 16)
     float o[6][4];
     forward<true>(m, sw, sx, o, zs, batch, b0);
     __syncwarp();
@@ -193,13 +199,18 @@ __global__ void __launch_bounds__(128) mlp_train_fb_kernel(MlpDev m, const float
         const int NT = layer_out(l) / 8;
         // transposed dz of layer l (weight gradient operand) and bias gradient
         __nv_bfloat16 *dst = m.dzT + (size_t)dz_row(l) * batch + b0;
+        uint32_t da[4][4];   // dZ as bf16 A fragments
+        #pragma unroll
+        for (int kt = 0; kt < NT / 2; ++kt) {
+            da[kt][0] = pack_bf16(dz[2 * kt][0], dz[2 * kt][1]);
+            da[kt][1] = pack_bf16(dz[2 * kt][2], dz[2 * kt][3]);
+            da[kt][2] = pack_bf16(dz[2 * kt + 1][0], dz[2 * kt + 1][1]);
+            da[kt][3] = pack_bf16(dz[2 * kt + 1][2], dz[2 * kt + 1][3]);
+            store_transposed_tile(dst, batch, kt * 16, da[kt]);
+        }
         #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
             const int c = nt * 8 + 2 * t;
-            dst[(size_t)c * batch + g] = __float2bfloat16(dz[nt][0]);
-            dst[(size_t)(c + 1) * batch + g] = __float2bfloat16(dz[nt][1]);
-            dst[(size_t)c * batch + g + 8] = __float2bfloat16(dz[nt][2]);
-            dst[(size_t)(c + 1) * batch + g + 8] = __float2bfloat16(dz[nt][3]);
             float s0 = dz[nt][0] + dz[nt][2], s1 = dz[nt][1] + dz[nt][3];
             #pragma unroll
             for (int off = 4; off < 32; off <<= 1) {
@@ -213,14 +224,6 @@ __global__ void __launch_bounds__(128) mlp_train_fb_kernel(MlpDev m, const float
         }
         if (l == 0) break;
         // dH_{l-1} = dZ_l W_l: A = dZ (bf16), B from the [in][out] copy
-        uint32_t da[4][4];
-        #pragma unroll
-        for (int kt = 0; kt < NT / 2; ++kt) {
-            da[kt][0] = pack_bf16(dz[2 * kt][0], dz[2 * kt][1]);
-            da[kt][1] = pack_bf16(dz[2 * kt][2], dz[2 * kt][3]);
-            da[kt][2] = pack_bf16(dz[2 * kt + 1][0], dz[2 * kt + 1][1]);
-            da[kt][3] = pack_bf16(dz[2 * kt + 1][2], dz[2 * kt + 1][3]);
-        }
         const __nv_bfloat16 *Wb = sw + smb_off(l);
         const int ldb = layer_out(l) + kPadK;
         const float *zp = zs + ((l - 1) * 8 * 4) * 32 + lane;
@@ -239,13 +242,20 @@ __global__ void __launch_bounds__(128) mlp_train_fb_kernel(MlpDev m, const float
     }
 }
 
+// Samples a warp of mlp_wgrad_kernel sums up (the last one of a tile fewer).
+// 8,192 samples at 128 / 256 / 512 / 1024: 113 / 110 / 111 / 112 us a gradient:
+// longer chunks leave warps idle, shorter ones add more atomics.  A chunk that
+// had to divide the batch was 32 samples at 31,712 (529 us, now 235).
+constexpr int kWgradChunk = 256;
+
 // dW_l[o][i] += sum_b dz_l[b][o] h_l[b][i] over one batch chunk; one warp per
-// (layer, 16x8 output tile, chunk).  A = dz^T rows, B = h^T rows: both read as
-// contiguous bf16 pairs along the batch.
-__global__ void __launch_bounds__(128) mlp_wgrad_kernel(MlpDev m, int batch, int chunk) {
+// (layer, 16x8 output tile, chunk).  A = dz^T rows, B = h^T rows, both
+// contiguous along the batch.  Bound by the latency of its loads, which are
+// 16 bytes a lane (4 bytes before: 23 -> 8 us at 8,192 samples).
+__global__ void __launch_bounds__(128) mlp_wgrad_kernel(MlpDev m, int batch) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int wid = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-    const int chunks = batch / chunk;
+    const int chunks = (batch + kWgradChunk - 1) / kWgradChunk;
     int tile = wid / chunks;
     const int ch = wid % chunks;
     int l = 0;
@@ -257,17 +267,30 @@ __global__ void __launch_bounds__(128) mlp_wgrad_kernel(MlpDev m, int batch, int
     if (l >= kLayers) return;
     const int K = layer_in(l);
     const int mt = tile / (K / 8), nt = tile % (K / 8);
-    const __nv_bfloat16 *dz = m.dzT + (size_t)dz_row(l) * batch;
-    const __nv_bfloat16 *h = m.hT + (size_t)h_row(l) * batch;
+    const int b0 = ch * kWgradChunk, len = min(kWgradChunk, batch - b0);   // a multiple of 16
+    const __nv_bfloat16 *ar = m.dzT + (size_t)(dz_row(l) + mt * 16 + g) * batch + b0;
+    const __nv_bfloat16 *ar8 = ar + (size_t)8 * batch;
+    const __nv_bfloat16 *br = m.hT + (size_t)(h_row(l) + nt * 8 + g) * batch + b0;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int bb = ch * chunk; bb < (ch + 1) * chunk; bb += 16) {
-        const __nv_bfloat16 *ar = dz + (size_t)(mt * 16 + g) * batch + bb + 2 * t;
-        const __nv_bfloat16 *ar8 = ar + (size_t)8 * batch;
-        const uint32_t a[4] = {*reinterpret_cast<const uint32_t *>(ar), *reinterpret_cast<const uint32_t *>(ar8),
-                               *reinterpret_cast<const uint32_t *>(ar + 8),
-                               *reinterpret_cast<const uint32_t *>(ar8 + 8)};
-        const __nv_bfloat16 *br = h + (size_t)(nt * 8 + g) * batch + bb + 2 * t;
-        mma16816(acc, a, *reinterpret_cast<const uint32_t *>(br), *reinterpret_cast<const uint32_t *>(br + 8));
+    // The order of the samples within the sum is free as long as A and B agree:
+    // lane t of a row takes 8 consecutive ones in one load, four pairs that
+    // serve as the k pairs of two products.  Rows start on 16 bytes (the batch
+    // is a multiple of 16 samples).
+    const int wide = len & ~31;
+    #pragma unroll 8
+    for (int bb = 8 * t; bb < wide; bb += 32) {
+        const uint4 a = *reinterpret_cast<const uint4 *>(ar + bb), a8 = *reinterpret_cast<const uint4 *>(ar8 + bb),
+                    bv = *reinterpret_cast<const uint4 *>(br + bb);
+        const uint32_t a0[4] = {a.x, a8.x, a.y, a8.y}, a1[4] = {a.z, a8.z, a.w, a8.w};
+        mma16816(acc, a0, bv.x, bv.y);
+        mma16816(acc, a1, bv.z, bv.w);
+    }
+    if (wide < len) {
+        const int bb = wide + 2 * t;
+        const uint32_t a[4] = {*reinterpret_cast<const uint32_t *>(ar + bb), *reinterpret_cast<const uint32_t *>(ar8 + bb),
+                               *reinterpret_cast<const uint32_t *>(ar + bb + 8),
+                               *reinterpret_cast<const uint32_t *>(ar8 + bb + 8)};
+        mma16816(acc, a, *reinterpret_cast<const uint32_t *>(br + bb), *reinterpret_cast<const uint32_t *>(br + bb + 8));
     }
     float *gw = m.grad + w_off(l);
     const int r0 = mt * 16 + g, c0 = nt * 8 + 2 * t;
@@ -370,21 +393,14 @@ cudaError_t launch_forward(const MlpDev &m, const float *feat, uint32_t n, float
     return cudaGetLastError();
 }
 
-static int wgrad_chunk(int batch) {
-    for (int c = 1024; c > 16; c >>= 1)
-        if (batch % c == 0) return c;
-    return 16;
-}
-
 cudaError_t launch_train_step(const MlpDev &m, const float *feat, const float *uv, size_t ld, uint32_t n_data,
                               int batch, float lr, bool shuffle, bool update, cudaStream_t s) {
     const int warps = batch / 16;
     mlp_train_fb_kernel<<<(warps + 3) / 4, 128, smem_train(), s>>>(m, feat, uv, ld, n_data, batch, shuffle ? 1 : 0);
     int tiles = 0;
     for (int l = 0; l < kLayers; ++l) tiles += (layer_out(l) / 16) * (layer_in(l) / 8);
-    const int chunk = wgrad_chunk(batch);
-    const int wg_warps = tiles * (batch / chunk);
-    mlp_wgrad_kernel<<<(wg_warps + 3) / 4, 128, 0, s>>>(m, batch, chunk);
+    const int wg_warps = tiles * ((batch + kWgradChunk - 1) / kWgradChunk);
+    mlp_wgrad_kernel<<<(wg_warps + 3) / 4, 128, 0, s>>>(m, batch);
     if (update) {
         mlp_adam_kernel<<<(kParams + 255) / 256, 256, 0, s>>>(m, lr);
         mlp_step_kernel<<<1, 1, 0, s>>>(m);

@@ -39,37 +39,65 @@ __device__ __forceinline__ float dsilu(float z) {
     return s * (1.f + z * (1.f - s));
 }
 
-// Copy bf16 weights (first `elems` elements) to shared memory; 16-byte moves.
+// Copy bf16 weights (first `elems` elements) to shared memory: 16-byte
+// asynchronous copies, all in flight at once; stage_wait before their use.
 __device__ __forceinline__ void stage_weights(const __nv_bfloat16 *__restrict__ src, __nv_bfloat16 *dst, int elems) {
-    const uint4 *s4 = reinterpret_cast<const uint4 *>(src);
-    uint4 *d4 = reinterpret_cast<uint4 *>(dst);
-    for (int i = threadIdx.x; i < elems / 8; i += blockDim.x) d4[i] = __ldg(s4 + i);
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    for (int i = threadIdx.x; i < elems / 8; i += blockDim.x)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16u * (uint32_t)i), "l"(src + 8 * i)
+                     : "memory");
+}
+__device__ __forceinline__ void stage_wait() {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+}
+
+// An 8x8 block of bf16 accumulator pairs (lane 4 g + t: row g, columns 2 t and
+// 2 t + 1) to its transpose in memory: columns c0 .. c0 + 7 are rows of `ld`
+// elements, its rows their elements r0 .. r0 + 7.
+__device__ __forceinline__ void store_transposed(__nv_bfloat16 *dst, size_t ld, int c0, int r0, uint32_t frag) {
+    const int lane = threadIdx.x & 31;
+    uint32_t tr;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(tr) : "r"(frag));
+    *reinterpret_cast<uint32_t *>(dst + (size_t)(c0 + (lane >> 2)) * ld + r0 + 2 * (lane & 3)) = tr;
+}
+__device__ __forceinline__ void store_transposed_tile(__nv_bfloat16 *dst, size_t ld, int c0, const uint32_t a[4]) {
+    store_transposed(dst, ld, c0, 0, a[0]);
+    store_transposed(dst, ld, c0, 8, a[1]);
+    store_transposed(dst, ld, c0 + 8, 0, a[2]);
+    store_transposed(dst, ld, c0 + 8, 8, a[3]);
 }
 
 // Stage the encoded inputs of a 16-row tile as bf16 rows of kXLd elements:
-// lanes 0..15 each write the row of their own normalised features xn (the
-// other lanes' xn is ignored).  Columns: xn[0..8], then per feature sin
+// lanes l and l + 16 write row l, from the row's normalised features xn on
+// both; half of the features each.  Columns: xn[0..8], then per feature sin
 // (pi 2^j xn), j < kEncFreq, and cos (pi 2^j xn), then zeros.
 __device__ __forceinline__ void stage_inputs(const float xn[kIn], __nv_bfloat16 *sx) {
     const int lane = threadIdx.x & 31;
-    if (lane < 16) {
-        __nv_bfloat16 *row = sx + lane * kXLd;
-        #pragma unroll
-        for (int f = 0; f < kIn; ++f) {
-            row[f] = __float2bfloat16(xn[f]);
+    __nv_bfloat16 *row = sx + (lane & 15) * kXLd;
+    constexpr int kHalf = (kIn + 1) / 2;
+    #pragma unroll
+    for (int k = 0; k < kHalf; ++k) {
+        const bool high = lane >= 16;
+        const int f = high ? k + kHalf : k;
+        const float x = high ? (k + kHalf < kIn ? xn[k + kHalf < kIn ? k + kHalf : 0] : 0.f) : xn[k];
+        if (f < kIn) {
+            row[f] = __float2bfloat16(x);
             #pragma unroll
             for (int j = 0; j < kEncFreq; ++j) {
                 float sn, cs;
-                sincospif(xn[f] * (float)(1 << j), &sn, &cs);
+                sincospif(x * (float)(1 << j), &sn, &cs);
                 row[kIn + f * 2 * kEncFreq + j] = __float2bfloat16(sn);
                 row[kIn + f * 2 * kEncFreq + kEncFreq + j] = __float2bfloat16(cs);
             }
+        } else {
+            #pragma unroll
+            for (int c = kInEnc; c < kInPad; ++c) row[c] = __float2bfloat16(0.f);
         }
-        #pragma unroll
-        for (int c = kInEnc; c < kInPad; ++c) row[c] = __float2bfloat16(0.f);
     }
     __syncwarp();
 }
+static_assert(2 * ((kIn + 1) / 2) == kIn + 1, "stage_inputs: the odd slot writes the padding");
 
 // Forward pass of one warp's 16 samples.  sw: forward weight copy in shared
 // memory; sx: the staged input tile.  out: accumulators of the output layer
@@ -80,13 +108,6 @@ template <bool kTrain>
 __device__ __forceinline__ void forward(const MlpDev &m, const __nv_bfloat16 *sw, const __nv_bfloat16 *sx,
                                         float out[6][4], float *zs = nullptr, int batch = 0, int b0 = 0) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    if (kTrain) {
-        // layer-0 input, transposed
-        for (int i = lane; i < kInPad * 16; i += 32) {
-            const int c = i >> 4, r = i & 15;
-            m.hT[(size_t)c * batch + b0 + r] = sx[r * kXLd + c];
-        }
-    }
     uint32_t a[4][4];
     #pragma unroll
     for (int l = 0; l < kLayers; ++l) {
@@ -95,19 +116,7 @@ __device__ __forceinline__ void forward(const MlpDev &m, const __nv_bfloat16 *sw
         if (kTrain && l > 0) {
             __nv_bfloat16 *dst = m.hT + (size_t)h_row(l) * batch + b0;
             #pragma unroll
-            for (int kt = 0; kt < 4; ++kt) {
-                const int k0 = kt * 16 + 2 * t;
-                const float2 v0 = unpack_bf16(a[kt][0]), v1 = unpack_bf16(a[kt][1]);
-                const float2 v2 = unpack_bf16(a[kt][2]), v3 = unpack_bf16(a[kt][3]);
-                dst[(size_t)k0 * batch + g] = __float2bfloat16(v0.x);
-                dst[(size_t)(k0 + 1) * batch + g] = __float2bfloat16(v0.y);
-                dst[(size_t)k0 * batch + g + 8] = __float2bfloat16(v1.x);
-                dst[(size_t)(k0 + 1) * batch + g + 8] = __float2bfloat16(v1.y);
-                dst[(size_t)(k0 + 8) * batch + g] = __float2bfloat16(v2.x);
-                dst[(size_t)(k0 + 9) * batch + g] = __float2bfloat16(v2.y);
-                dst[(size_t)(k0 + 8) * batch + g + 8] = __float2bfloat16(v3.x);
-                dst[(size_t)(k0 + 9) * batch + g + 8] = __float2bfloat16(v3.y);
-            }
+            for (int kt = 0; kt < 4; ++kt) store_transposed_tile(dst, batch, kt * 16, a[kt]);
         }
         float acc[8][4];
         #pragma unroll
@@ -124,6 +133,7 @@ __device__ __forceinline__ void forward(const MlpDev &m, const __nv_bfloat16 *sw
                                         *reinterpret_cast<const uint32_t *>(xp + 8 * kXLd),
                                         *reinterpret_cast<const uint32_t *>(xp + 8),
                                         *reinterpret_cast<const uint32_t *>(xp + 8 * kXLd + 8)};
+                if (kTrain) store_transposed_tile(m.hT + b0, batch, kt * 16, a0);
                 #pragma unroll
                 for (int nt = 0; nt < NT; ++nt) {
                     const __nv_bfloat16 *wp = W + (nt * 8 + g) * ld + kt * 16 + 2 * t;

@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(128, 3) ss_proposal_kernel(DevScene sc, Solver
                    (threadIdx.x / 32) * (32 * mlp::kIn + kStage);
     float *stage = feats + 32 * mlp::kIn;
     mlp::stage_weights(pr.net.wbf, sw, mlp::kWeightsFwd);
-    __syncthreads();
+    mlp::stage_wait();
     const unsigned lane = threadIdx.x & 31;
     const uint32_t wpb = blockDim.x / 32;
     for (uint32_t w = blockIdx.x * wpb + threadIdx.x / 32; (size_t)w * 32 < n; w += gridDim.x * wpb) {
