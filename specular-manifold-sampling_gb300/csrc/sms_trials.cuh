@@ -35,9 +35,10 @@ constexpr int kTrialOpen = 0x7fffffff;
 // Lists of at most this many grids' worth of trials run in a single pass.  A
 // pass of first trials costs one walk's latency (0.25 ms); what it saves is the
 // speculative trials of the queries that succeed at once.  Pane of 30,000
-// points (15,153 listed, 64 trials, 5.5 grids of 9 blocks per SM): one pass
-// 1.07 ms, two passes 1.34 ms; slab of 20,011 points (14,529 listed, 128
-// trials, 32 grids of 3 blocks): two passes 4.0 ms, one pass 4.5 ms.
+// points (15,153 listed, 64 trials, 12 grids of 4 blocks per SM): one pass
+// 0.76 ms, two passes 0.74 ms (1.07 and 1.34 ms when its grid had 9 blocks);
+// slab of 20,011 points (14,529 listed, 128 trials, 32 grids of 3 blocks): two
+// passes 3.2 ms, one pass 3.6 ms.
 constexpr unsigned kTrialSinglePass = 16;
 
 // Trials [lo, hi] of one pass, and the lanes of a warp that take part (`most`
