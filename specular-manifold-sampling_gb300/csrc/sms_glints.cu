@@ -196,7 +196,7 @@ SMS_D bool glint_walk(const DevScene &sc, const SolverCfg &cfg, const GQuery &q,
         }
         f2 prop = {uv.x - cfg.step_scale * beta * sx, uv.y - cfg.step_scale * beta * sy};
         it++;
-        if (!(inside_triangle(prop, fa, fb, fc) || inside_triangle(prop, fa, fc, fd))) {
+        if (!(inside_triangle(prop, fa, fb, fc) | inside_triangle(prop, fa, fc, fd))) {
             beta = 0.5f * beta;
             moved = false;
             continue;

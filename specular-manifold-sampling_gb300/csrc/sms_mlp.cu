@@ -44,45 +44,46 @@ __device__ __forceinline__ uint32_t hash32(uint32_t x) {
 }
 
 // Negative log-likelihood of (u, v) (relative to the anchor) under the
-// mixture of raw outputs o[40] and its gradient with respect to o (go[0..47],
-// padded columns zero).
-__device__ float mixture_nll(const float *o, float u, float v, float *go) {
-    float mx = o[0];
+// mixture of raw outputs row[40]; row becomes `scale` times its gradient with
+// respect to them (padded columns zero).
+__device__ float mixture_nll(float *row, float u, float v, float scale) {
+    float mx = row[0];
     #pragma unroll
-    for (int k = 1; k < kComp; ++k) mx = fmaxf(mx, o[k]);
+    for (int k = 1; k < kComp; ++k) mx = fmaxf(mx, row[k]);
     float se = 0.f;
     #pragma unroll
-    for (int k = 0; k < kComp; ++k) se += __expf(o[k] - mx);
+    for (int k = 0; k < kComp; ++k) se += __expf(row[k] - mx);
     const float logz = mx + __logf(se);
-    float lp[kComp], lmax = -INFINITY;
-    #pragma unroll
+    float *lp = row + kGmmParams;   // log densities, in the padding
+    static_assert(kOutPad - kGmmParams >= kComp, "the padding holds the log densities");
+    float lmax = -INFINITY;
+    #pragma unroll 2
     for (int k = 0; k < kComp; ++k) {
-        const float lsx = log_sigma(o[24 + 2 * k]), lsy = log_sigma(o[25 + 2 * k]);
-        const float dx = (u - o[8 + 2 * k]) * __expf(-lsx), dy = (v - o[9 + 2 * k]) * __expf(-lsy);
-        lp[k] = (o[k] - logz) - 1.8378770664093453f - lsx - lsy - 0.5f * (dx * dx + dy * dy);
+        const float lsx = log_sigma(row[24 + 2 * k]), lsy = log_sigma(row[25 + 2 * k]);
+        const float dx = (u - row[8 + 2 * k]) * __expf(-lsx), dy = (v - row[9 + 2 * k]) * __expf(-lsy);
+        lp[k] = (row[k] - logz) - 1.8378770664093453f - lsx - lsy - 0.5f * (dx * dx + dy * dy);
         lmax = fmaxf(lmax, lp[k]);
     }
     float s = 0.f;
     #pragma unroll
     for (int k = 0; k < kComp; ++k) s += __expf(lp[k] - lmax);
     const float logp = lmax + __logf(s);
-    #pragma unroll
+    #pragma unroll 2
     for (int k = 0; k < kComp; ++k) {
         const float r = __expf(lp[k] - logp);   // responsibility
-        go[k] = __expf(o[k] - logz) - r;
+        row[k] = (__expf(row[k] - logz) - r) * scale;
         #pragma unroll
         for (int d = 0; d < 2; ++d) {
-            const float raw = o[24 + 2 * k + d];
+            const float raw = row[24 + 2 * k + d];
             const float sg = sigmoid(raw);
             const float ls = kLsMin + (kLsMax - kLsMin) * sg;
             const float iv = __expf(-2.f * ls);
-            const float e = (d == 0 ? u : v) - o[8 + 2 * k + d];
-            go[8 + 2 * k + d] = -r * e * iv;
-            go[24 + 2 * k + d] = r * (1.f - e * e * iv) * (kLsMax - kLsMin) * sg * (1.f - sg);
+            const float e = (d == 0 ? u : v) - row[8 + 2 * k + d];
+            row[8 + 2 * k + d] = (-r * e * iv) * scale;
+            row[24 + 2 * k + d] = (r * (1.f - e * e * iv) * (kLsMax - kLsMin) * sg * (1.f - sg)) * scale;
         }
+        lp[k] = 0.f;
     }
-    #pragma unroll
-    for (int c = kGmmParams; c < kOutPad; ++c) go[c] = 0.f;
     return -logp;
 }
 
@@ -128,6 +129,51 @@ __global__ void __launch_bounds__(128) mlp_forward_kernel(MlpDev m, const float 
 }
 
 // ------------------------------------------------------------------ training
+// dz of layer l (NT n-tiles): its bf16 A fragments, its transposed copy (the
+// weight gradient's operand) and the bias gradient.
+template <int NT>
+__device__ __forceinline__ void dz_out(const MlpDev &m, const float dz[][4], uint32_t da[4][4], int l, int batch,
+                                       int b0) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    pack_tiles<NT / 2>(dz, da);
+    __nv_bfloat16 *dst = m.dzT + (size_t)dz_row(l) * batch + b0;
+    #pragma unroll
+    for (int kt = 0; kt < NT / 2; ++kt) store_transposed_tile(dst, batch, kt * 16, da[kt]);
+    float *gb = m.grad + b_off(l);
+    #pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+        const int c = nt * 8 + 2 * t;
+        float s0 = dz[nt][0] + dz[nt][2], s1 = dz[nt][1] + dz[nt][3];
+        #pragma unroll
+        for (int off = 4; off < 32; off <<= 1) {
+            s0 += __shfl_xor_sync(0xffffffffu, s0, off);
+            s1 += __shfl_xor_sync(0xffffffffu, s1, off);
+        }
+        if (g == 0) {
+            atomicAdd(gb + c, s0);
+            atomicAdd(gb + c + 1, s1);
+        }
+    }
+}
+
+// dz of the layer below: (dZ W) dsilu(z), W from the [in][out] copy with rows
+// of ldb elements, z the layer's pre-activations.
+template <int NT>
+__device__ __forceinline__ void dz_back(const __nv_bfloat16 *Wb, int ldb, const uint32_t da[4][4], const float *z,
+                                        float dz[8][4]) {
+    const int lane = threadIdx.x & 31;
+    #pragma unroll
+    for (int nt = 0; nt < 8; ++nt)
+        #pragma unroll
+        for (int i = 0; i < 4; ++i) dz[nt][i] = 0.f;
+    #pragma unroll
+    for (int kt = 0; kt < NT / 2; ++kt) mma_row<8>(Wb, ldb, kt, da[kt], dz);
+    #pragma unroll
+    for (int nt = 0; nt < 8; ++nt)
+        #pragma unroll
+        for (int i = 0; i < 4; ++i) dz[nt][i] *= dsilu(z[(nt * 4 + i) * 32 + lane]);
+}
+
 // A serial chain per warp, one warp per scheduler and block per SM (shared
 // memory): bound by its latency, 44 us at 8,192 samples (91 -> 67 us from a cold
 // cache).  The weights come asynchronously while the inputs are encoded, both
@@ -167,18 +213,13 @@ __global__ void __launch_bounds__(128) mlp_train_fb_kernel(MlpDev m, const float
     __syncwarp();
     float loss = 0.f;
     if (lane < 16) {
-        float oo[kOutPad], go[kOutPad];
-        #pragma unroll
-        for (int c = 0; c < kOutPad; ++c) oo[c] = stage[lane * kOutPad + c];
         const uint32_t r = row_of(lane);
         auto F = [&](int k) { return __ldg(feat + (size_t)k * ld + r); };
         float au, av;
         anchor_uv(m.frame, mk(F(0), F(1), F(2)), mk(F(3), F(4), F(5)), au, av);
-        loss = mixture_nll(oo, __ldg(uv + r) - au, __ldg(uv + ld + r) - av, go);
         // the loss is the batch mean of (weighted) NLLs
         const float inv_b = (m.weighted ? __ldg(uv + 2 * ld + r) : 1.f) / (float)batch;
-        #pragma unroll
-        for (int c = 0; c < kOutPad; ++c) stage[lane * kOutPad + c] = go[c] * inv_b;
+        loss = mixture_nll(stage + lane * kOutPad, __ldg(uv + r) - au, __ldg(uv + ld + r) - av, inv_b);
         loss *= inv_b;
     }
     #pragma unroll
@@ -194,53 +235,20 @@ __global__ void __launch_bounds__(128) mlp_train_fb_kernel(MlpDev m, const float
         dz[nt][2] = stage[(g + 8) * kOutPad + c];
         dz[nt][3] = stage[(g + 8) * kOutPad + c + 1];
     }
-    #pragma unroll
-    for (int l = kLayers - 1; l >= 0; --l) {
-        const int NT = layer_out(l) / 8;
-        // transposed dz of layer l (weight gradient operand) and bias gradient
-        __nv_bfloat16 *dst = m.dzT + (size_t)dz_row(l) * batch + b0;
-        uint32_t da[4][4];   // dZ as bf16 A fragments
-        #pragma unroll
-        for (int kt = 0; kt < NT / 2; ++kt) {
-            da[kt][0] = pack_bf16(dz[2 * kt][0], dz[2 * kt][1]);
-            da[kt][1] = pack_bf16(dz[2 * kt][2], dz[2 * kt][3]);
-            da[kt][2] = pack_bf16(dz[2 * kt + 1][0], dz[2 * kt + 1][1]);
-            da[kt][3] = pack_bf16(dz[2 * kt + 1][2], dz[2 * kt + 1][3]);
-            store_transposed_tile(dst, batch, kt * 16, da[kt]);
-        }
-        #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-            const int c = nt * 8 + 2 * t;
-            float s0 = dz[nt][0] + dz[nt][2], s1 = dz[nt][1] + dz[nt][3];
-            #pragma unroll
-            for (int off = 4; off < 32; off <<= 1) {
-                s0 += __shfl_xor_sync(0xffffffffu, s0, off);
-                s1 += __shfl_xor_sync(0xffffffffu, s1, off);
-            }
-            if (g == 0) {
-                atomicAdd(m.grad + b_off(l) + c, s0);
-                atomicAdd(m.grad + b_off(l) + c + 1, s1);
-            }
-        }
-        if (l == 0) break;
-        // dH_{l-1} = dZ_l W_l: A = dZ (bf16), B from the [in][out] copy
-        const __nv_bfloat16 *Wb = sw + smb_off(l);
-        const int ldb = layer_out(l) + kPadK;
-        const float *zp = zs + ((l - 1) * 8 * 4) * 32 + lane;
-        #pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-            float dh[4] = {0.f, 0.f, 0.f, 0.f};
-            #pragma unroll
-            for (int kt = 0; kt < NT / 2; ++kt) {
-                const __nv_bfloat16 *wp = Wb + (nt * 8 + g) * ldb + kt * 16 + 2 * t;
-                mma16816(dh, da[kt], *reinterpret_cast<const uint32_t *>(wp),
-                         *reinterpret_cast<const uint32_t *>(wp + 8));
-            }
-            #pragma unroll
-            for (int i = 0; i < 4; ++i) dz[nt][i] = dh[i] * dsilu(zp[(nt * 4 + i) * 32]);
-        }
+    // dz of the output layer, then of the hidden layers in a loop
+    uint32_t da[4][4];
+    dz_out<6>(m, dz, da, kLayers - 1, batch, b0);
+    dz_back<6>(sw + smb_off(kLayers - 1), layer_out(kLayers - 1) + kPadK, da, zs + (kLayers - 2) * 8 * 4 * 32, dz);
+    #pragma unroll 1
+    for (int l = kLayers - 2; l > 0; --l) {
+        dz_out<8>(m, dz, da, l, batch, b0);
+        dz_back<8>(sw + smb_off(1) + (l - 1) * kHidden * (kHidden + kPadK), kHidden + kPadK, da,
+                   zs + (l - 1) * 8 * 4 * 32, dz);
     }
+    dz_out<8>(m, dz, da, 0, batch, b0);
 }
+static_assert(smb_off(kLayers - 1) == smb_off(1) + (kLayers - 2) * kHidden * (kHidden + kPadK),
+              "hidden layers are evenly spaced");
 
 // Samples a warp of mlp_wgrad_kernel sums up (the last one of a tile fewer).
 // 8,192 samples at 128 / 256 / 512 / 1024: 113 / 110 / 111 / 112 us a gradient:

@@ -83,7 +83,7 @@ __device__ __forceinline__ void stage_inputs(const float xn[kIn], __nv_bfloat16 
         const float x = high ? (k + kHalf < kIn ? xn[k + kHalf < kIn ? k + kHalf : 0] : 0.f) : xn[k];
         if (f < kIn) {
             row[f] = __float2bfloat16(x);
-            #pragma unroll
+            #pragma unroll 1
             for (int j = 0; j < kEncFreq; ++j) {
                 float sn, cs;
                 sincospif(x * (float)(1 << j), &sn, &cs);
@@ -99,84 +99,97 @@ __device__ __forceinline__ void stage_inputs(const float xn[kIn], __nv_bfloat16 
 }
 static_assert(2 * ((kIn + 1) / 2) == kIn + 1, "stage_inputs: the odd slot writes the padding");
 
+// Accumulators of NT n-tiles, started from the bias.
+template <int NT>
+__device__ __forceinline__ void start_bias(const float *bias, float acc[][4]) {
+    const int t = threadIdx.x & 3;
+    #pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+        const float b0 = bias[nt * 8 + 2 * t], b1 = bias[nt * 8 + 2 * t + 1];
+        acc[nt][0] = b0; acc[nt][1] = b1; acc[nt][2] = b0; acc[nt][3] = b1;
+    }
+}
+
+// acc += A (one k-tile) x B, B rows of ld elements from W.
+template <int NT>
+__device__ __forceinline__ void mma_row(const __nv_bfloat16 *W, int ld, int kt, const uint32_t a[4], float acc[][4]) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    #pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+        const __nv_bfloat16 *wp = W + (nt * 8 + g) * ld + kt * 16 + 2 * t;
+        mma16816(acc[nt], a, *reinterpret_cast<const uint32_t *>(wp), *reinterpret_cast<const uint32_t *>(wp + 8));
+    }
+}
+
+// The accumulators of 2 KT n-tiles as KT bf16 A fragments.
+template <int KT>
+__device__ __forceinline__ void pack_tiles(const float acc[][4], uint32_t a[][4]) {
+    #pragma unroll
+    for (int kt = 0; kt < KT; ++kt) {
+        a[kt][0] = pack_bf16(acc[2 * kt][0], acc[2 * kt][1]);
+        a[kt][1] = pack_bf16(acc[2 * kt][2], acc[2 * kt][3]);
+        a[kt][2] = pack_bf16(acc[2 * kt + 1][0], acc[2 * kt + 1][1]);
+        a[kt][3] = pack_bf16(acc[2 * kt + 1][2], acc[2 * kt + 1][3]);
+    }
+}
+
 // Forward pass of one warp's 16 samples.  sw: forward weight copy in shared
 // memory; sx: the staged input tile.  out: accumulators of the output layer
 // (6 n-tiles).  When kTrain, the layer inputs are written transposed to hT
 // ([row][batch]) and the hidden pre-activations to zs (per warp,
 // [layer][ntile][4][32] floats).
+// The layers are a loop: a warp runs through this code once, and unrolled
+// (10,000 instructions in training) it waited for instructions more than for
+// anything else (7.5 of 13 cycles an instruction; FBMS).
 template <bool kTrain>
 __device__ __forceinline__ void forward(const MlpDev &m, const __nv_bfloat16 *sw, const __nv_bfloat16 *sx,
                                         float out[6][4], float *zs = nullptr, int batch = 0, int b0 = 0) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    float acc[8][4];
     uint32_t a[4][4];
-    #pragma unroll
-    for (int l = 0; l < kLayers; ++l) {
-        const int NT = layer_out(l) / 8, ld = layer_in(l) + kPadK;
-        const __nv_bfloat16 *W = sw + smf_off(l);
-        if (kTrain && l > 0) {
+    start_bias<8>(m.bias, acc);
+    // A fragments straight from the staged rows, one k-tile at a time
+    #pragma unroll 1
+    for (int kt = 0; kt < kInPad / 16; ++kt) {
+        const __nv_bfloat16 *xp = sx + g * kXLd + kt * 16 + 2 * t;
+        const uint32_t a0[4] = {*reinterpret_cast<const uint32_t *>(xp),
+                                *reinterpret_cast<const uint32_t *>(xp + 8 * kXLd),
+                                *reinterpret_cast<const uint32_t *>(xp + 8),
+                                *reinterpret_cast<const uint32_t *>(xp + 8 * kXLd + 8)};
+        if (kTrain) store_transposed_tile(m.hT + b0, batch, kt * 16, a0);
+        mma_row<8>(sw, kInPad + kPadK, kt, a0, acc);
+    }
+    #pragma unroll 1
+    for (int l = 1;; ++l) {
+        // acc: pre-activations of layer l - 1
+        #pragma unroll
+        for (int nt = 0; nt < 8; ++nt) {
+            if (kTrain) {
+                float *zp = zs + (((l - 1) * 8 + nt) * 4) * 32 + lane;
+                #pragma unroll
+                for (int i = 0; i < 4; ++i) zp[i * 32] = acc[nt][i];
+            }
+            #pragma unroll
+            for (int i = 0; i < 4; ++i) acc[nt][i] = silu(acc[nt][i]);
+        }
+        pack_tiles<4>(acc, a);
+        if (kTrain) {
             __nv_bfloat16 *dst = m.hT + (size_t)h_row(l) * batch + b0;
             #pragma unroll
             for (int kt = 0; kt < 4; ++kt) store_transposed_tile(dst, batch, kt * 16, a[kt]);
         }
-        float acc[8][4];
+        if (l == kLayers - 1) break;
+        const __nv_bfloat16 *W = sw + smf_off(1) + (l - 1) * kHidden * (kHidden + kPadK);
+        start_bias<8>(m.bias + l * 64, acc);
         #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-            const float bb0 = m.bias[l * 64 + nt * 8 + 2 * t], bb1 = m.bias[l * 64 + nt * 8 + 2 * t + 1];
-            acc[nt][0] = bb0; acc[nt][1] = bb1; acc[nt][2] = bb0; acc[nt][3] = bb1;
-        }
-        if (l == 0) {
-            // A fragments straight from the staged rows, one k-tile at a time
-            #pragma unroll
-            for (int kt = 0; kt < kInPad / 16; ++kt) {
-                const __nv_bfloat16 *xp = sx + g * kXLd + kt * 16 + 2 * t;
-                const uint32_t a0[4] = {*reinterpret_cast<const uint32_t *>(xp),
-                                        *reinterpret_cast<const uint32_t *>(xp + 8 * kXLd),
-                                        *reinterpret_cast<const uint32_t *>(xp + 8),
-                                        *reinterpret_cast<const uint32_t *>(xp + 8 * kXLd + 8)};
-                if (kTrain) store_transposed_tile(m.hT + b0, batch, kt * 16, a0);
-                #pragma unroll
-                for (int nt = 0; nt < NT; ++nt) {
-                    const __nv_bfloat16 *wp = W + (nt * 8 + g) * ld + kt * 16 + 2 * t;
-                    mma16816(acc[nt], a0, *reinterpret_cast<const uint32_t *>(wp),
-                             *reinterpret_cast<const uint32_t *>(wp + 8));
-                }
-            }
-        } else {
-            #pragma unroll
-            for (int nt = 0; nt < NT; ++nt)
-                #pragma unroll
-                for (int kt = 0; kt < 4; ++kt) {
-                    const __nv_bfloat16 *wp = W + (nt * 8 + g) * ld + kt * 16 + 2 * t;
-                    mma16816(acc[nt], a[kt], *reinterpret_cast<const uint32_t *>(wp),
-                             *reinterpret_cast<const uint32_t *>(wp + 8));
-                }
-        }
-        if (l == kLayers - 1) {
-            #pragma unroll
-            for (int nt = 0; nt < 6; ++nt)
-                #pragma unroll
-                for (int i = 0; i < 4; ++i) out[nt][i] = acc[nt][i];
-        } else {
-            #pragma unroll
-            for (int nt = 0; nt < 8; ++nt) {
-                if (kTrain) {
-                    float *zp = zs + ((l * 8 + nt) * 4) * 32 + lane;
-                    #pragma unroll
-                    for (int i = 0; i < 4; ++i) zp[i * 32] = acc[nt][i];
-                }
-                #pragma unroll
-                for (int i = 0; i < 4; ++i) acc[nt][i] = silu(acc[nt][i]);
-            }
-            #pragma unroll
-            for (int kt = 0; kt < 4; ++kt) {
-                a[kt][0] = pack_bf16(acc[2 * kt][0], acc[2 * kt][1]);
-                a[kt][1] = pack_bf16(acc[2 * kt][2], acc[2 * kt][3]);
-                a[kt][2] = pack_bf16(acc[2 * kt + 1][0], acc[2 * kt + 1][1]);
-                a[kt][3] = pack_bf16(acc[2 * kt + 1][2], acc[2 * kt + 1][3]);
-            }
-        }
+        for (int kt = 0; kt < 4; ++kt) mma_row<8>(W, kHidden + kPadK, kt, a[kt], acc);
     }
+    start_bias<6>(m.bias + (kLayers - 1) * 64, out);
+    #pragma unroll
+    for (int kt = 0; kt < 4; ++kt) mma_row<6>(sw + smf_off(kLayers - 1), kHidden + kPadK, kt, a[kt], out);
 }
+static_assert(smf_off(kLayers - 1) == smf_off(1) + (kLayers - 2) * kHidden * (kHidden + kPadK),
+              "hidden layers are evenly spaced");
 
 // Write the output accumulators as rows of `stage` ([16][kOutPad] floats).
 __device__ __forceinline__ void stage_outputs(const float o[6][4], float *stage) {
