@@ -12,7 +12,7 @@
 //
 // One optimizer step is four launches:
 //   mlp_train_fb_kernel  forward, mixture NLL and its gradient, backward
-//                        through all layers (register-resident per warp);
+//                        through all layers (two warps per 16 samples);
 //                        writes the transposed layer inputs h^T and
 //                        pre-activation gradients dz^T, accumulates bias
 //                        gradients and the batch loss
@@ -27,11 +27,15 @@
 namespace sms {
 namespace mlp {
 
-constexpr int kZsFloats = 4 * 8 * 4 * 32;   // per warp: hidden pre-activations
-// per warp: the staged input tile (16 x kXLd bf16), reused for the output
+constexpr int kZsFloats = 4 * 8 * 4 * 32;   // per 16 samples: hidden pre-activations
+// per 16 samples: the staged input tile (16 x kXLd bf16), reused for the output
 // rows (16 x kOutPad floats)
 constexpr int kStageFloats = 16 * kXLd / 2;
 static_assert(kStageFloats >= 16 * kOutPad, "stage holds the output rows");
+// training, per 16 samples: the A fragments its two warps pass each other,
+// [buffer][k-tile][register][lane]
+constexpr int kPassWords = 2 * 4 * 4 * 32;
+constexpr int kTrainTiles = 4;   // 16-sample tiles of a training block
 
 // lowbias32 integer hash (C. Wellons, "Prospecting for hash functions").
 __device__ __forceinline__ uint32_t hash32(uint32_t x) {
@@ -108,7 +112,7 @@ __global__ void __launch_bounds__(128) mlp_forward_kernel(MlpDev m, const float 
         __nv_bfloat16 *sx = reinterpret_cast<__nv_bfloat16 *>(stage);
         stage_inputs(xn, sx);
         float o[6][4];
-        forward<false>(m, sw, sx, o);
+        forward(m, sw, sx, o);
         __syncwarp();
         stage_outputs(o, stage);
         __syncwarp();
@@ -129,17 +133,45 @@ __global__ void __launch_bounds__(128) mlp_forward_kernel(MlpDev m, const float 
 }
 
 // ------------------------------------------------------------------ training
-// dz of layer l (NT n-tiles): its bf16 A fragments, its transposed copy (the
-// weight gradient's operand) and the bias gradient.
+// A serial chain per 16 samples, one block per SM (shared memory): bound by the
+// latency of its instructions.  Two warps share the 16 samples, each with half
+// of every layer's outputs, and pass each other their halves as bf16 A
+// fragments (8,192 samples: 42 us with one warp, 33 with two).  The layers are a
+// loop: the code is run through once, and unrolled (10,000 instructions) its warps
+// waited more for instructions than for anything else (from a cold cache 7.5 of 13
+// cycles an instruction; now 0.1 of 7).  The weights come asynchronously while the
+// inputs are encoded.
+struct TrainTile {
+    uint32_t *pass;   // kPassWords
+    int tile, half;   // of the block; this warp's half of the outputs
+    int turn = 0;     // buffer of the next exchange
+
+    __device__ __forceinline__ void sync() const {
+        asm volatile("bar.sync %0, 64;" ::"r"(1 + tile) : "memory");
+    }
+    // own: this warp's k-tiles 2 half and 2 half + 1; a: all four.  The buffers
+    // alternate, so that a warp may write the next before the other has read
+    // this one, and only that.
+    __device__ __forceinline__ void exchange(const uint32_t own[2][4], uint32_t a[4][4]) {
+        const int lane = threadIdx.x & 31;
+        uint32_t *buf = pass + turn * (kPassWords / 2) + lane;
+        turn ^= 1;
+        #pragma unroll
+        for (int k = 0; k < 2; ++k)
+            #pragma unroll
+            for (int i = 0; i < 4; ++i) buf[((2 * half + k) * 4 + i) * 32] = own[k][i];
+        sync();
+        #pragma unroll
+        for (int k = 0; k < 4; ++k)
+            #pragma unroll
+            for (int i = 0; i < 4; ++i) a[k][i] = buf[(k * 4 + i) * 32];
+    }
+};
+
+// Bias gradient of NT n-tiles of dz, gb the first one's.
 template <int NT>
-__device__ __forceinline__ void dz_out(const MlpDev &m, const float dz[][4], uint32_t da[4][4], int l, int batch,
-                                       int b0) {
+__device__ __forceinline__ void bias_grad(const float dz[][4], float *gb) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    pack_tiles<NT / 2>(dz, da);
-    __nv_bfloat16 *dst = m.dzT + (size_t)dz_row(l) * batch + b0;
-    #pragma unroll
-    for (int kt = 0; kt < NT / 2; ++kt) store_transposed_tile(dst, batch, kt * 16, da[kt]);
-    float *gb = m.grad + b_off(l);
     #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
         const int c = nt * 8 + 2 * t;
@@ -156,40 +188,39 @@ __device__ __forceinline__ void dz_out(const MlpDev &m, const float dz[][4], uin
     }
 }
 
-// dz of the layer below: (dZ W) dsilu(z), W from the [in][out] copy with rows
-// of ldb elements, z the layer's pre-activations.
-template <int NT>
+// This warp's half of the dz of the layer below: (dZ W) dsilu(z), W its rows of
+// the [in][out] copy (ldb elements each), z its pre-activations.
+template <int KT>
 __device__ __forceinline__ void dz_back(const __nv_bfloat16 *Wb, int ldb, const uint32_t da[4][4], const float *z,
-                                        float dz[8][4]) {
+                                        float dz[4][4]) {
     const int lane = threadIdx.x & 31;
     #pragma unroll
-    for (int nt = 0; nt < 8; ++nt)
+    for (int nt = 0; nt < 4; ++nt)
         #pragma unroll
         for (int i = 0; i < 4; ++i) dz[nt][i] = 0.f;
     #pragma unroll
-    for (int kt = 0; kt < NT / 2; ++kt) mma_row<8>(Wb, ldb, kt, da[kt], dz);
+    for (int kt = 0; kt < KT; ++kt) mma_row<4>(Wb, ldb, kt, da[kt], dz);
     #pragma unroll
-    for (int nt = 0; nt < 8; ++nt)
+    for (int nt = 0; nt < 4; ++nt)
         #pragma unroll
         for (int i = 0; i < 4; ++i) dz[nt][i] *= dsilu(z[(nt * 4 + i) * 32 + lane]);
 }
 
-// A serial chain per warp, one warp per scheduler and block per SM (shared
-// memory): bound by its latency, 44 us at 8,192 samples (91 -> 67 us from a cold
-// cache).  The weights come asynchronously while the inputs are encoded, both
-// halves of the warp encode, and the fragments leave transposed, two samples a
-// store.
-__global__ void __launch_bounds__(128) mlp_train_fb_kernel(MlpDev m, const float *__restrict__ feat,
-                                                           const float *__restrict__ uv, size_t ld, uint32_t n_data,
-                                                           int batch, int shuffle) {
+__global__ void __launch_bounds__(64 * kTrainTiles) mlp_train_fb_kernel(MlpDev m, const float *__restrict__ feat,
+                                                                        const float *__restrict__ uv, size_t ld,
+                                                                        uint32_t n_data, int batch, int shuffle) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __nv_bfloat16 *sw = reinterpret_cast<__nv_bfloat16 *>(smem_raw);
-    float *zs = reinterpret_cast<float *>(smem_raw + (size_t)kWeightsAll * 2) + (threadIdx.x / 32) * kZsFloats;
-    float *stage = reinterpret_cast<float *>(smem_raw + (size_t)kWeightsAll * 2) + 4 * kZsFloats +
-                   (threadIdx.x / 32) * kStageFloats;
+    float *fsm = reinterpret_cast<float *>(smem_raw + (size_t)kWeightsAll * 2);
+    TrainTile T;
+    T.tile = (int)(threadIdx.x / 64);
+    T.half = (int)(threadIdx.x / 32) & 1;
+    float *zs = fsm + T.tile * kZsFloats;
+    float *stage = fsm + kTrainTiles * kZsFloats + T.tile * kStageFloats;
+    T.pass = reinterpret_cast<uint32_t *>(fsm + kTrainTiles * (kZsFloats + kStageFloats)) + T.tile * kPassWords;
     stage_weights(m.wbf, sw, kWeightsAll);
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int b0 = (blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32) * 16;
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, half = T.half;
+    const int b0 = ((int)blockIdx.x * kTrainTiles + T.tile) * 16;
     const uint32_t step = *m.step;
     auto row_of = [&](int r) -> uint32_t {
         const uint32_t b = (uint32_t)(b0 + r);
@@ -197,55 +228,120 @@ __global__ void __launch_bounds__(128) mlp_train_fb_kernel(MlpDev m, const float
     };
     __nv_bfloat16 *sx = reinterpret_cast<__nv_bfloat16 *>(stage);
     if (b0 < batch) {
-        // while the weights come
-        float xn[kIn];
+        // while the weights come: a quarter of the features per 16 lanes
         const uint32_t r = row_of(lane & 15);
+        __nv_bfloat16 *row = sx + (lane & 15) * kXLd;
+        const int q = 2 * half + (lane >> 4);
         #pragma unroll
-        for (int k = 0; k < kIn; ++k) xn[k] = (__ldg(feat + (size_t)k * ld + r) - m.shift[k]) * m.scale[k];
-        stage_inputs(xn, sx);
+        for (int k = 0; k < (kIn + 3) / 4; ++k) {
+            const int f = q + 4 * k;
+            if (f < kIn) stage_feature(row, f, (__ldg(feat + (size_t)f * ld + r) - m.shift[f]) * m.scale[f]);
+        }
+        if (q == 3) stage_padding(row);
     }
     stage_wait();
-    if (b0 >= batch) return;   // whole warps only (batch is a multiple of 16)
-    float o[6][4];
-    forward<true>(m, sw, sx, o, zs, batch, b0);
-    __syncwarp();
-    stage_outputs(o, stage);
-    __syncwarp();
+    if (b0 >= batch) return;   // whole tiles only (batch is a multiple of 16)
+
+    // ---- forward
+    float acc[4][4];
+    uint32_t own[2][4], a[4][4];
+    const int n0 = 32 * half;   // first output of this warp
+    start_bias<4>(m.bias + n0, acc);
+    #pragma unroll 1
+    for (int kt = 0; kt < kInPad / 16; ++kt) {
+        uint32_t a0[4];
+        input_fragment(sx, kt, a0);
+        if ((kt & 1) == half) store_transposed_tile(m.hT + b0, batch, kt * 16, a0);
+        mma_row<4>(sw + n0 * (kInPad + kPadK), kInPad + kPadK, kt, a0, acc);
+    }
+    #pragma unroll 1
+    for (int l = 1;; ++l) {
+        // acc: pre-activations of layer l - 1
+        float *zp = zs + (((l - 1) * 8 + 4 * half) * 4) * 32 + lane;
+        #pragma unroll
+        for (int nt = 0; nt < 4; ++nt)
+            #pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                zp[(nt * 4 + i) * 32] = acc[nt][i];
+                acc[nt][i] = silu(acc[nt][i]);
+            }
+        pack_tiles<2>(acc, own);
+        __nv_bfloat16 *dst = m.hT + (size_t)h_row(l) * batch + b0;
+        store_transposed_tile(dst, batch, n0, own[0]);
+        store_transposed_tile(dst, batch, n0 + 16, own[1]);
+        T.exchange(own, a);
+        if (l == kLayers - 1) break;
+        const __nv_bfloat16 *W = sw + smf_off(1) + ((l - 1) * kHidden + n0) * (kHidden + kPadK);
+        start_bias<4>(m.bias + l * 64 + n0, acc);
+        #pragma unroll
+        for (int kt = 0; kt < 4; ++kt) mma_row<4>(W, kHidden + kPadK, kt, a[kt], acc);
+    }
+    {
+        float o[3][4];
+        start_bias<3>(m.bias + (kLayers - 1) * 64 + 24 * half, o);
+        #pragma unroll
+        for (int kt = 0; kt < 4; ++kt)
+            mma_row<3>(sw + smf_off(kLayers - 1) + 24 * half * (kHidden + kPadK), kHidden + kPadK, kt, a[kt], o);
+        // the inputs under the output rows were last read before the exchanges
+        stage_outputs<3>(o, stage, 24 * half);
+    }
+    T.sync();
+
+    // ---- loss, 8 rows a warp
     float loss = 0.f;
-    if (lane < 16) {
-        const uint32_t r = row_of(lane);
+    if (lane < 8) {
+        const int i = 8 * half + lane;
+        const uint32_t r = row_of(i);
         auto F = [&](int k) { return __ldg(feat + (size_t)k * ld + r); };
         float au, av;
         anchor_uv(m.frame, mk(F(0), F(1), F(2)), mk(F(3), F(4), F(5)), au, av);
         // the loss is the batch mean of (weighted) NLLs
         const float inv_b = (m.weighted ? __ldg(uv + 2 * ld + r) : 1.f) / (float)batch;
-        loss = mixture_nll(stage + lane * kOutPad, __ldg(uv + r) - au, __ldg(uv + ld + r) - av, inv_b);
-        loss *= inv_b;
+        loss = mixture_nll(stage + i * kOutPad, __ldg(uv + r) - au, __ldg(uv + ld + r) - av, inv_b) * inv_b;
     }
     #pragma unroll
     for (int off = 16; off > 0; off >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, off);
     if (lane == 0) atomicAdd(m.loss + step % kLossHist, loss);
-    __syncwarp();
-    float dz[8][4];
-    #pragma unroll
-    for (int nt = 0; nt < 6; ++nt) {
-        const int c = nt * 8 + 2 * t;
-        dz[nt][0] = stage[g * kOutPad + c];
-        dz[nt][1] = stage[g * kOutPad + c + 1];
-        dz[nt][2] = stage[(g + 8) * kOutPad + c];
-        dz[nt][3] = stage[(g + 8) * kOutPad + c + 1];
+    T.sync();
+
+    // ---- backward: dz of the output layer whole on both warps, then halves
+    {
+        float dz[6][4];
+        #pragma unroll
+        for (int nt = 0; nt < 6; ++nt) {
+            const int c = nt * 8 + 2 * t;
+            dz[nt][0] = stage[g * kOutPad + c];
+            dz[nt][1] = stage[g * kOutPad + c + 1];
+            dz[nt][2] = stage[(g + 8) * kOutPad + c];
+            dz[nt][3] = stage[(g + 8) * kOutPad + c + 1];
+        }
+        pack_tiles<3>(dz, a);
+        __nv_bfloat16 *dst = m.dzT + (size_t)dz_row(kLayers - 1) * batch + b0;
+        float *gb = m.grad + b_off(kLayers - 1);
+        if (half == 0) {
+            store_transposed_tile(dst, batch, 0, a[0]);
+            store_transposed_tile(dst, batch, 16, a[1]);
+            bias_grad<2>(dz, gb);
+        } else {
+            store_transposed_tile(dst, batch, 32, a[2]);
+            bias_grad<4>(dz + 2, gb + 16);
+        }
     }
-    // dz of the output layer, then of the hidden layers in a loop
-    uint32_t da[4][4];
-    dz_out<6>(m, dz, da, kLayers - 1, batch, b0);
-    dz_back<6>(sw + smb_off(kLayers - 1), layer_out(kLayers - 1) + kPadK, da, zs + (kLayers - 2) * 8 * 4 * 32, dz);
+    dz_back<3>(sw + smb_off(kLayers - 1) + n0 * (kOutPad + kPadK), kOutPad + kPadK, a,
+               zs + ((kLayers - 2) * 8 + 4 * half) * 4 * 32, acc);
     #pragma unroll 1
-    for (int l = kLayers - 2; l > 0; --l) {
-        dz_out<8>(m, dz, da, l, batch, b0);
-        dz_back<8>(sw + smb_off(1) + (l - 1) * kHidden * (kHidden + kPadK), kHidden + kPadK, da,
-                   zs + (l - 1) * 8 * 4 * 32, dz);
+    for (int l = kLayers - 2;; --l) {
+        pack_tiles<2>(acc, own);
+        __nv_bfloat16 *dst = m.dzT + (size_t)dz_row(l) * batch + b0;
+        store_transposed_tile(dst, batch, n0, own[0]);
+        store_transposed_tile(dst, batch, n0 + 16, own[1]);
+        if (l == 0) break;
+        T.exchange(own, a);
+        bias_grad<4>(acc, m.grad + b_off(l) + n0);
+        dz_back<4>(sw + smb_off(1) + ((l - 1) * kHidden + n0) * (kHidden + kPadK), kHidden + kPadK, a,
+                   zs + ((l - 1) * 8 + 4 * half) * 4 * 32, acc);
     }
-    dz_out<8>(m, dz, da, 0, batch, b0);
+    bias_grad<4>(acc, m.grad + b_off(0) + n0);
 }
 static_assert(smb_off(kLayers - 1) == smb_off(1) + (kLayers - 2) * kHidden * (kHidden + kPadK),
               "hidden layers are evenly spaced");
@@ -377,7 +473,9 @@ __global__ void feature_moments_kernel(const float *__restrict__ feat, size_t ld
 
 // ---------------------------------------------------------------- launchers
 size_t smem_forward() { return (size_t)kWeightsFwd * 2 + (size_t)4 * kStageFloats * 4; }
-size_t smem_train() { return (size_t)kWeightsAll * 2 + (size_t)4 * (kZsFloats + kStageFloats) * 4; }
+size_t smem_train() {
+    return (size_t)kWeightsAll * 2 + (size_t)kTrainTiles * (kZsFloats + kStageFloats + kPassWords) * 4;
+}
 size_t smem_seed_fused() { return (size_t)kWeightsFwd * 2 + (size_t)4 * (32 * kIn + kStageFloats) * 4; }
 
 cudaError_t configure_kernels() {
@@ -403,8 +501,8 @@ cudaError_t launch_forward(const MlpDev &m, const float *feat, uint32_t n, float
 
 cudaError_t launch_train_step(const MlpDev &m, const float *feat, const float *uv, size_t ld, uint32_t n_data,
                               int batch, float lr, bool shuffle, bool update, cudaStream_t s) {
-    const int warps = batch / 16;
-    mlp_train_fb_kernel<<<(warps + 3) / 4, 128, smem_train(), s>>>(m, feat, uv, ld, n_data, batch, shuffle ? 1 : 0);
+    mlp_train_fb_kernel<<<(batch / 16 + kTrainTiles - 1) / kTrainTiles, 64 * kTrainTiles, smem_train(), s>>>(
+        m, feat, uv, ld, n_data, batch, shuffle ? 1 : 0);
     int tiles = 0;
     for (int l = 0; l < kLayers; ++l) tiles += (layer_out(l) / 16) * (layer_in(l) / 8);
     const int wg_warps = tiles * ((batch + kWgradChunk - 1) / kWgradChunk);

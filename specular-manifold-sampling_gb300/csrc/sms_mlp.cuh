@@ -68,10 +68,26 @@ __device__ __forceinline__ void store_transposed_tile(__nv_bfloat16 *dst, size_t
     store_transposed(dst, ld, c0 + 8, 8, a[3]);
 }
 
+// Feature f = x of a row of the staged input tile: columns xn[0..8], then per
+// feature sin (pi 2^j xn), j < kEncFreq, and cos (pi 2^j xn), then zeros.
+__device__ __forceinline__ void stage_feature(__nv_bfloat16 *row, int f, float x) {
+    row[f] = __float2bfloat16(x);
+    #pragma unroll 1
+    for (int j = 0; j < kEncFreq; ++j) {
+        float sn, cs;
+        sincospif(x * (float)(1 << j), &sn, &cs);
+        row[kIn + f * 2 * kEncFreq + j] = __float2bfloat16(sn);
+        row[kIn + f * 2 * kEncFreq + kEncFreq + j] = __float2bfloat16(cs);
+    }
+}
+__device__ __forceinline__ void stage_padding(__nv_bfloat16 *row) {
+    #pragma unroll
+    for (int c = kInEnc; c < kInPad; ++c) row[c] = __float2bfloat16(0.f);
+}
+
 // Stage the encoded inputs of a 16-row tile as bf16 rows of kXLd elements:
 // lanes l and l + 16 write row l, from the row's normalised features xn on
-// both; half of the features each.  Columns: xn[0..8], then per feature sin
-// (pi 2^j xn), j < kEncFreq, and cos (pi 2^j xn), then zeros.
+// both; half of the features each.
 __device__ __forceinline__ void stage_inputs(const float xn[kIn], __nv_bfloat16 *sx) {
     const int lane = threadIdx.x & 31;
     __nv_bfloat16 *row = sx + (lane & 15) * kXLd;
@@ -79,25 +95,23 @@ __device__ __forceinline__ void stage_inputs(const float xn[kIn], __nv_bfloat16 
     #pragma unroll
     for (int k = 0; k < kHalf; ++k) {
         const bool high = lane >= 16;
-        const int f = high ? k + kHalf : k;
         const float x = high ? (k + kHalf < kIn ? xn[k + kHalf < kIn ? k + kHalf : 0] : 0.f) : xn[k];
-        if (f < kIn) {
-            row[f] = __float2bfloat16(x);
-            #pragma unroll 1
-            for (int j = 0; j < kEncFreq; ++j) {
-                float sn, cs;
-                sincospif(x * (float)(1 << j), &sn, &cs);
-                row[kIn + f * 2 * kEncFreq + j] = __float2bfloat16(sn);
-                row[kIn + f * 2 * kEncFreq + kEncFreq + j] = __float2bfloat16(cs);
-            }
-        } else {
-            #pragma unroll
-            for (int c = kInEnc; c < kInPad; ++c) row[c] = __float2bfloat16(0.f);
-        }
+        if (high && k + kHalf >= kIn) stage_padding(row);
+        else stage_feature(row, high ? k + kHalf : k, x);
     }
     __syncwarp();
 }
 static_assert(2 * ((kIn + 1) / 2) == kIn + 1, "stage_inputs: the odd slot writes the padding");
+
+// A fragment kt of the staged input rows.
+__device__ __forceinline__ void input_fragment(const __nv_bfloat16 *sx, int kt, uint32_t a[4]) {
+    const int lane = threadIdx.x & 31;
+    const __nv_bfloat16 *xp = sx + (lane >> 2) * kXLd + kt * 16 + 2 * (lane & 3);
+    a[0] = *reinterpret_cast<const uint32_t *>(xp);
+    a[1] = *reinterpret_cast<const uint32_t *>(xp + 8 * kXLd);
+    a[2] = *reinterpret_cast<const uint32_t *>(xp + 8);
+    a[3] = *reinterpret_cast<const uint32_t *>(xp + 8 * kXLd + 8);
+}
 
 // Accumulators of NT n-tiles, started from the bias.
 template <int NT>
@@ -135,54 +149,31 @@ __device__ __forceinline__ void pack_tiles(const float acc[][4], uint32_t a[][4]
 
 // Forward pass of one warp's 16 samples.  sw: forward weight copy in shared
 // memory; sx: the staged input tile.  out: accumulators of the output layer
-// (6 n-tiles).  When kTrain, the layer inputs are written transposed to hT
-// ([row][batch]) and the hidden pre-activations to zs (per warp,
-// [layer][ntile][4][32] floats).
-// The layers are a loop: a warp runs through this code once, and unrolled
-// (10,000 instructions in training) it waited for instructions more than for
-// anything else (7.5 of 13 cycles an instruction; FBMS).
-template <bool kTrain>
+// (6 n-tiles).  The layers are a loop (see mlp_train_fb_kernel).
 __device__ __forceinline__ void forward(const MlpDev &m, const __nv_bfloat16 *sw, const __nv_bfloat16 *sx,
-                                        float out[6][4], float *zs = nullptr, int batch = 0, int b0 = 0) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+                                        float out[6][4]) {
     float acc[8][4];
     uint32_t a[4][4];
     start_bias<8>(m.bias, acc);
-    // A fragments straight from the staged rows, one k-tile at a time
     #pragma unroll 1
     for (int kt = 0; kt < kInPad / 16; ++kt) {
-        const __nv_bfloat16 *xp = sx + g * kXLd + kt * 16 + 2 * t;
-        const uint32_t a0[4] = {*reinterpret_cast<const uint32_t *>(xp),
-                                *reinterpret_cast<const uint32_t *>(xp + 8 * kXLd),
-                                *reinterpret_cast<const uint32_t *>(xp + 8),
-                                *reinterpret_cast<const uint32_t *>(xp + 8 * kXLd + 8)};
-        if (kTrain) store_transposed_tile(m.hT + b0, batch, kt * 16, a0);
+        uint32_t a0[4];
+        input_fragment(sx, kt, a0);
         mma_row<8>(sw, kInPad + kPadK, kt, a0, acc);
     }
     #pragma unroll 1
     for (int l = 1;; ++l) {
         // acc: pre-activations of layer l - 1
         #pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-            if (kTrain) {
-                float *zp = zs + (((l - 1) * 8 + nt) * 4) * 32 + lane;
-                #pragma unroll
-                for (int i = 0; i < 4; ++i) zp[i * 32] = acc[nt][i];
-            }
+        for (int nt = 0; nt < 8; ++nt)
             #pragma unroll
             for (int i = 0; i < 4; ++i) acc[nt][i] = silu(acc[nt][i]);
-        }
         pack_tiles<4>(acc, a);
-        if (kTrain) {
-            __nv_bfloat16 *dst = m.hT + (size_t)h_row(l) * batch + b0;
-            #pragma unroll
-            for (int kt = 0; kt < 4; ++kt) store_transposed_tile(dst, batch, kt * 16, a[kt]);
-        }
         if (l == kLayers - 1) break;
-        const __nv_bfloat16 *W = sw + smf_off(1) + (l - 1) * kHidden * (kHidden + kPadK);
         start_bias<8>(m.bias + l * 64, acc);
         #pragma unroll
-        for (int kt = 0; kt < 4; ++kt) mma_row<8>(W, kHidden + kPadK, kt, a[kt], acc);
+        for (int kt = 0; kt < 4; ++kt)
+            mma_row<8>(sw + smf_off(1) + (l - 1) * kHidden * (kHidden + kPadK), kHidden + kPadK, kt, a[kt], acc);
     }
     start_bias<6>(m.bias + (kLayers - 1) * 64, out);
     #pragma unroll
@@ -191,12 +182,14 @@ __device__ __forceinline__ void forward(const MlpDev &m, const __nv_bfloat16 *sw
 static_assert(smf_off(kLayers - 1) == smf_off(1) + (kLayers - 2) * kHidden * (kHidden + kPadK),
               "hidden layers are evenly spaced");
 
-// Write the output accumulators as rows of `stage` ([16][kOutPad] floats).
-__device__ __forceinline__ void stage_outputs(const float o[6][4], float *stage) {
+// Write the accumulators of NT n-tiles of the output layer from column c0 on as
+// rows of `stage` ([16][kOutPad] floats).
+template <int NT = 6>
+__device__ __forceinline__ void stage_outputs(const float o[][4], float *stage, int c0 = 0) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     #pragma unroll
-    for (int nt = 0; nt < 6; ++nt) {
-        const int c = nt * 8 + 2 * t;
+    for (int nt = 0; nt < NT; ++nt) {
+        const int c = c0 + nt * 8 + 2 * t;
         stage[g * kOutPad + c] = o[nt][0];
         stage[g * kOutPad + c + 1] = o[nt][1];
         stage[(g + 8) * kOutPad + c] = o[nt][2];

@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(128, 3) ss_proposal_kernel(DevScene sc, Solver
             __nv_bfloat16 *sx = reinterpret_cast<__nv_bfloat16 *>(stage);
             mlp::stage_inputs(xn, sx);
             float o[6][4];
-            mlp::forward<false>(pr.net, sw, sx, o);
+            mlp::forward(pr.net, sw, sx, o);
             __syncwarp();
             mlp::stage_outputs(o, stage);
             __syncwarp();
