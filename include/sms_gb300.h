@@ -655,7 +655,10 @@ uint64_t sms_render_sms_seed(uint64_t seed);
  * normal-mapped BSDF samples its nested BSDF in the frame of the bilinear
  * slope normal elsewhere (normalmap.cpp:118-135).
  * The LEAN pyramid (5 floats per texel over all levels, 4/3 x 20 bytes per
- * texel of the slope map) is built on the device at the first glint render. */
+ * texel of the slope map) is built on the device at the first glint render.
+ *
+ * The context keeps the render's device buffers (up to 1 GiB) for its next
+ * render and frees them when it is destroyed. */
 sms_status sms_render(sms_ctx *ctx, const sms_camera *cam, const sms_render_options *opt, float *image);
 sms_status sms_render_device(sms_ctx *ctx, const sms_camera *cam, const sms_render_options *opt,
                              float *image_dev);
