@@ -10,11 +10,14 @@
 //                      query of a receiver vertex (staged, not solved), emitter
 //                      sampling with MIS, BSDF sampling, the next intersection
 //                      and the emitter it hits (filtered like the reference,
-//                      with the unbiased-MNEE check walk of path_sms_ss)
-//   pt_scan_kernel     ordered prefix sum of the per-block query counts
-//   pt_gather_kernel   appends the staged queries of this bounce to the
-//                      wavefront's pending SMS batch, in path order, each
-//                      with its random-number stream (path, bounce)
+//                      with the unbiased-MNEE check walk of path_sms_ss); the
+//                      last paths of integrators without queries to their ends
+//   pt_scan_kernel     ordered prefix sums of the per-block counts of queries
+//                      and live paths
+//   pt_gather_kernel   lists the live paths for the next bounce and appends the
+//                      staged queries of this one to the wavefront's pending
+//                      SMS batch, both in path order, each query with its
+//                      random-number stream (path, bounce)
 //   pt_pack_kernel     the pending batch as one SoA query array
 //   (SMS estimator)    the context's single- or multi-scatter connection
 //                      kernels on the whole pending batch: the queries of all
