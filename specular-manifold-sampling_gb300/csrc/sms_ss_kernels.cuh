@@ -35,12 +35,26 @@ namespace sms {
 // two-stage solver at 4 / 5 / 6 / 9 blocks: 0.76 / 0.80 / 0.91 / 1.06 ms.
 constexpr int ss_walk_blocks(int var) { return (var & 4) ? 4 : SMS_SS_WALK_MIN_BLOCKS; }
 
+// The same of the biased estimator's kernel for large batches (see below), and
+// the blocks per SM from which a batch is large.  4 / 6 / 8 blocks, biased:
+//   sphere, 13,355 points x 32 walks (22 blocks per SM)     374 / 348 / 376 us
+//   sphere, 3,745 x 24 (6)                                  130 / 136 / 127 us
+//   water 256^2, 16,000 x 32 (26)                           4.7 / 3.8 ms
+//   pane, two-stage, 82,185 x 64 (135)                      22.4 / 19.8 / 18.5 ms
+//   pane, two-stage, 11,000 x 16 (9); 12,000 x 32 (20)      0.48 / - / 0.55; 1.36 / - / 1.38 ms
+//   pane, one stage, 51,728 x 64 (85)                       4.9 / 5.0 / 5.0 ms
+constexpr int ss_biased_blocks(int var) { return var == 0 ? 6 : var == 6 ? 8 : 4; }
+constexpr uint32_t ss_biased_large(int var) { return var == 0 ? 8u : 32u; }
+
 // ------------------------------------------------------ biased estimator
 // Group of G lanes per query; walk m of caster c sits at stream position
 // 3 + 2 (c M + m).  Contributions are summed in walk order over the first
 // occurrences of each solution direction, exactly as manifold_ss.cpp:146-196.
-template <int G, int kVar>
-__global__ void __launch_bounds__(128, 4) ss_biased_kernel(DevScene sc, SolverCfg cfg, const float *__restrict__ qs,
+// Compiled for kBlocks resident blocks per SM (128 threads): 4 hold the Newton
+// step in registers, which is what counts while the batch fits the chip; more
+// hide more of its latency in larger batches (ss_biased_blocks).
+template <int G, int kVar, int kBlocks>
+__global__ void __launch_bounds__(128, kBlocks) ss_biased_kernel(DevScene sc, SolverCfg cfg, const float *__restrict__ qs,
                                                         uint32_t n, uint64_t seed, uint64_t stream_off,
                                                         float *__restrict__ value, int *__restrict__ count,
                                                         int *__restrict__ walks, DevCounters *ctr) {
@@ -340,7 +354,10 @@ cudaError_t ss_biased_launch(const DevScene &sc, const SolverCfg &cfg, const flo
     uint32_t blocks_needed = (n + groups_per_block - 1) / groups_per_block;
     uint32_t blocks = std::min<uint32_t>(blocks_needed, (uint32_t)(num_sms * bps));
     phase_begin(tm, kPhaseSsBiased, s);
-    auto biased = G == 16 ? ss_biased_kernel<16, kVar> : ss_biased_kernel<32, kVar>;
+    constexpr int kMany = ss_biased_blocks(kVar);
+    const bool many = kMany > 4 && blocks_needed > ss_biased_large(kVar) * (uint32_t)num_sms;
+    auto biased = G == 16 ? (many ? ss_biased_kernel<16, kVar, kMany> : ss_biased_kernel<16, kVar, 4>)
+                          : (many ? ss_biased_kernel<32, kVar, kMany> : ss_biased_kernel<32, kVar, 4>);
     biased<<<blocks, 128, 0, s>>>(sc, cfg, q, n, seed, stream_off, value, count, walks, ctr);
     phase_end(tm, s);
     return cudaGetLastError();
