@@ -471,7 +471,7 @@ def learned_study(torch, sms, W, ctx, dev, pairs=4 << 20, steps=20000, batch=819
     ws = torch.empty(ns, dtype=torch.int32, device=f"cuda:{dev}")
     torch.cuda.synchronize()
     tune = autotune_ss(sms, ctx, qs.data_ptr(), ns, vs.data_ptr(), cs.data_ptr(), ws.data_ptr(),
-                       blocks_per_sm=(16,), trial_groups=(8, 16, 32), treelets=(0,), chunks=(1,), seed=99)
+                       blocks_per_sm=(0,), trial_groups=(8, 16, 32), treelets=(0,), chunks=(1,), seed=99)
     learned_group = tune["best"][1]
     ctx.set_proposal(None)
     ctx.set_launch(0, 0)

@@ -1,13 +1,14 @@
 """Launch-shape autotuner of the SMS solvers.
 
 Picks, for one context and a representative device-resident query sample,
-the persistent kernels' blocks per SM (warps per SM = 4 x blocks), the
-Bernoulli-trial group size (trials run side by side per query = walks in
-flight per query), the number of top tree nodes the trial kernel stages in
-shared memory, and the queries a lane group claims from the trial queue per
-atomic (queue chunk); for the multi-scatter and glint estimators, blocks per
-SM.  Each candidate is timed with the library's own CUDA-event phase profile
-(sms_profile_read).  No candidate changes a result: the random
+the persistent kernels' blocks per SM (warps per SM = 4 x blocks), the lanes
+of a warp of the Bernoulli-trial kernel that take trials (trial group), the
+number of top tree nodes the trial kernel stages in shared memory, and the
+rounds of trials a warp claims from the stream per atomic (queue chunk); for
+the multi-scatter and glint estimators, blocks per SM.  The library's own
+blocks per SM (0), which differ from kernel to kernel, are among the
+candidates.  Each candidate is timed with the library's own CUDA-event phase
+profile (sms_profile_read).  No candidate changes a result: the random
 numbers of every walk are fixed by the query's stream, so only speed is
 compared.
 """
@@ -29,7 +30,7 @@ def _time_ss(ss, ctx, args, seed, repeats):
 
 
 def autotune_ss(sms, ctx, queries_ptr: int, n: int, value_ptr: int, count_ptr: int, walks_ptr: int,
-                blocks_per_sm=(2, 4, 6, 8, 12, 16), trial_groups=(8, 16, 32), treelets=(0, 64, 128, 256, 384),
+                blocks_per_sm=(0, 2, 4, 6, 8, 12, 16), trial_groups=(8, 16, 32), treelets=(0, 64, 128, 256, 384),
                 chunks=(1, 2, 4), seed: int = 12345, repeats: int = 2) -> dict:
     """Time every (blocks_per_sm, trial_group) pair on the sample (device
     pointers, as SpecularManifoldSingleScatter.specular_manifold_sampling_device),
@@ -72,7 +73,7 @@ def autotune_ss(sms, ctx, queries_ptr: int, n: int, value_ptr: int, count_ptr: i
 
 
 def autotune_blocks(sms, ctx, kind: str, queries_ptr: int, n: int, value_ptr: int, count_ptr: int, walks_ptr: int,
-                    blocks_per_sm=(2, 4, 6, 8, 12, 16), seed: int = 12345, repeats: int = 2) -> dict:
+                    blocks_per_sm=(0, 2, 4, 6, 8, 12, 16), seed: int = 12345, repeats: int = 2) -> dict:
     """Blocks per SM of the multi-scatter ("ms") or glint ("glints") kernels,
     timed with their phase of the CUDA-event profile on a device-resident
     sample; sets the fastest on ctx and returns {"best": bps, "ms": {...}}."""
