@@ -96,16 +96,17 @@ struct TrialStream {
                 const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x / 32);
                 const unsigned long long share = total / (4 * warps) / plan.lanes;
                 const unsigned claim = (unsigned)plan.lanes * (unsigned)max((unsigned long long)chunk, min(4ull, max(1ull, share)));
-                unsigned long long got = 0;
-                unsigned done = 0;
-                if (lane == 0) {
+                // Once every query has a success the warp stops, and it looks
+                // before it claims: a claimed range is never dropped, because it
+                // can hold a trial before a success that another warp found in
+                // a later range in the meantime.  All ranges before a success
+                // then belong to warps that run them.
+                unsigned long long got = total;
+                if (lane == 0 && *(volatile unsigned *)&ctr->trial_done < n_list)
                     got = atomicAdd(&ctr->trial_jobs[pass], (unsigned long long)claim);
-                    done = *(volatile unsigned *)&ctr->trial_done;
-                }
                 cur = __shfl_sync(full, got, 0);
-                done = __shfl_sync(full, done, 0);
                 end = min(cur + claim, total);
-                if (cur >= total || done >= n_list) { drained = true; break; }
+                if (cur >= total) { drained = true; break; }
             }
             const int k = (int)min((unsigned long long)plan.lanes, end - cur);
             bool open = false;
