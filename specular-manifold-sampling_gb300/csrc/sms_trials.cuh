@@ -148,12 +148,9 @@ struct TrialStream {
 // Record the end of trial t of query qi.
 SMS_D void trial_end(int *count, DevCounters *ctr, uint32_t qi, int t, bool succ, int it, LaneStats &st) {
     st.spec++;   // the trials up to each query's first success are taken out at the end
-    if (succ) {
-        if (atomicMin(count + qi, t) == kTrialOpen) atomicAdd(&ctr->trial_done, 1u);
-        st.newton += (unsigned)it;
-    } else if (*(volatile const int *)(count + qi) > t) {
-        st.newton += (unsigned)it;
-    }
+    const int before = succ ? atomicMin(count + qi, t) : *(volatile const int *)(count + qi);   // the success known so far
+    if (succ && before == kTrialOpen) atomicAdd(&ctr->trial_done, 1u);
+    if (before > t) st.newton += (unsigned)it;
 }
 
 // The estimate's trial statistics once all trials have run: f the first
