@@ -658,7 +658,8 @@ uint64_t sms_render_sms_seed(uint64_t seed);
  * texel of the slope map) is built on the device at the first glint render.
  *
  * The context keeps the render's device buffers (up to 1 GiB) for its next
- * render and frees them when it is destroyed. */
+ * render.  They are freed when it is destroyed, and when an allocation of any
+ * context or proposal on the device would fail without them. */
 sms_status sms_render(sms_ctx *ctx, const sms_camera *cam, const sms_render_options *opt, float *image);
 sms_status sms_render_device(sms_ctx *ctx, const sms_camera *cam, const sms_render_options *opt,
                              float *image_dev);

@@ -10,7 +10,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
-#include <mutex>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -512,8 +512,7 @@ struct sms_ctx {
     // estimator only: rough multi-scatter chain shapes / glinty shapes
     bool ms_rough = false, glint_rough = false;
     bool ms_nm = false;   // a multi-scatter chain shape carries the normal map
-    std::mutex render_mutex;   // guards render_buf
-    RenderBuffers render_buf;  // of the last render, kept for the next (ctx_give_render)
+    std::unique_ptr<RenderKeep> render_keep;   // the last render's buffers, for the next
     uint32_t render_spp = 0;   // samples per pixel of the last render
     bool nm_rough = false;   // the normal-mapped shape is rough
     float *lean = nullptr;   // LEAN pyramid of the slope map (glints integrator), built on first use
@@ -524,7 +523,7 @@ static sms_status upload(sms_ctx *c, const std::vector<T> &v, const T **out) {
     *out = nullptr;
     if (v.empty()) return SMS_OK;
     void *p = nullptr;
-    CUDA_TRY(cudaMalloc(&p, v.size() * sizeof(T)));
+    CUDA_TRY(device_malloc(&p, v.size() * sizeof(T)));
     c->allocs.push_back(p);
     CUDA_TRY(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, c->stream));
     *out = reinterpret_cast<const T *>(p);
@@ -562,8 +561,7 @@ extern "C" void sms_ctx_destroy(sms_ctx *c) {
     if (c->io) cudaFree(c->io);
     if (c->scratch) cudaFree(c->scratch);
     if (c->lean) cudaFree(c->lean);
-    if (c->render_buf.block) cudaFree(c->render_buf.block);
-    if (c->render_buf.host) cudaFreeHost(c->render_buf.host);
+    c->render_keep.reset();
     if (c->ms_tmpl) cudaFree(c->ms_tmpl);
     if (c->gmm) cudaFree(c->gmm);
     for (sms_proposal *p : c->proposals) proposal_detach(p);
@@ -799,13 +797,14 @@ extern "C" sms_status sms_ctx_create(const sms_scene *s, const sms_config *cfg, 
     sms_ctx *c = new sms_ctx();
     c->device = device;
     c->cfg = *cfg;
+    c->render_keep.reset(new RenderKeep(device));
     sms_status st = SMS_OK;
     do {
         cudaError_t e = cudaSetDevice(device);
         if (e != cudaSuccess) { st = cuda_fail(e, "cudaSetDevice"); break; }
         e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
         if (e != cudaSuccess) { st = cuda_fail(e, "cudaStreamCreate"); break; }
-        e = cudaMalloc(&c->ctr, sizeof(DevCounters));
+        e = device_malloc(reinterpret_cast<void **>(&c->ctr), sizeof(DevCounters));
         if (e != cudaSuccess) { st = cuda_fail(e, "cudaMalloc(counters)"); break; }
         e = cudaMemsetAsync(c->ctr, 0, sizeof(DevCounters), c->stream);
         if (e != cudaSuccess) { st = cuda_fail(e, "cudaMemset(counters)"); break; }
@@ -939,7 +938,7 @@ static sms_status ensure_scratch(sms_ctx *c, uint32_t n, SsScratch &scr) {
             c->scratch = nullptr;
             c->scratch_n = 0;
         }
-        CUDA_TRY(cudaMalloc(&c->scratch, ss_scratch_bytes(n)));
+        CUDA_TRY(device_malloc(&c->scratch, ss_scratch_bytes(n)));
         c->scratch_n = n;
     }
     char *b = reinterpret_cast<char *>(c->scratch);
@@ -1012,7 +1011,7 @@ sms_status ctx_ss_connect(sms_ctx *c, const float *q, uint32_t n, uint64_t seed,
                 c->gmm = nullptr;
                 c->gmm_n = 0;
             }
-            CUDA_TRY(cudaMalloc(&c->gmm, (size_t)mlp::kGmmParams * n * sizeof(float)));
+            CUDA_TRY(device_malloc(reinterpret_cast<void **>(&c->gmm), (size_t)mlp::kGmmParams * n * sizeof(float)));
             c->gmm_n = n;
         }
         if (!proposal_seed_desc(c->prop, pr)) return fail(SMS_ERR_INVALID_ARG, "proposal is not usable");
@@ -1067,7 +1066,7 @@ static sms_status ensure_io(sms_ctx *c, size_t bytes) {
         c->io = nullptr;
         c->io_bytes = 0;
     }
-    CUDA_TRY(cudaMalloc(&c->io, bytes));
+    CUDA_TRY(device_malloc(&c->io, bytes));
     c->io_bytes = bytes;
     return SMS_OK;
 }
@@ -1204,7 +1203,8 @@ sms_status ctx_ms_connect(sms_ctx *c, const float *q, uint32_t n, uint64_t seed,
             }
             // template shapes (kMaxBounces rows), then the template's offset
             // normals (3 kMaxBounces rows) and their density (1 row)
-            CUDA_TRY(cudaMalloc(&c->ms_tmpl, (size_t)(4 * kMaxBounces + 1) * n * sizeof(int)));
+            CUDA_TRY(device_malloc(reinterpret_cast<void **>(&c->ms_tmpl),
+                                   (size_t)(4 * kMaxBounces + 1) * n * sizeof(int)));
             c->ms_tmpl_n = n;
         }
     }
@@ -1312,44 +1312,9 @@ extern "C" sms_status sms_glint_connect_batch_device(sms_ctx *c, const float *q,
     return ctx_glint_connect(c, q, n, seed, stream_off, nullptr, out);
 }
 
-// A render's path state (643 MB for the default wavefront with SMS queries) and
-// its pinned words took 0.8 ms to allocate and free, as long as a small image
-// takes to render.
-constexpr size_t kRenderKeepBytes = (size_t)1 << 30;
+cudaError_t ctx_take_render(sms_ctx *c, size_t bytes, RenderBuffers &out) { return c->render_keep->take(bytes, out); }
 
-cudaError_t ctx_take_render(sms_ctx *c, size_t bytes, RenderBuffers &out) {
-    {
-        std::lock_guard<std::mutex> lock(c->render_mutex);
-        out = c->render_buf;
-        c->render_buf = RenderBuffers{};
-    }
-    cudaError_t e = cudaSuccess;
-    if (out.bytes < bytes) {
-        if (out.block) cudaFree(out.block);
-        out.block = nullptr;
-        out.bytes = 0;
-        e = cudaMalloc(&out.block, bytes);
-        if (e == cudaSuccess) out.bytes = bytes;
-    }
-    if (e == cudaSuccess && !out.host) e = cudaMallocHost(&out.host, 2 * sizeof(uint32_t));
-    return e;
-}
-
-void ctx_give_render(sms_ctx *c, RenderBuffers &buf) {
-    if (buf.bytes > kRenderKeepBytes) {
-        cudaFree(buf.block);
-        buf.block = nullptr;
-        buf.bytes = 0;
-    }
-    {
-        // the larger block stays
-        std::lock_guard<std::mutex> lock(c->render_mutex);
-        if (buf.bytes >= c->render_buf.bytes) std::swap(buf, c->render_buf);
-    }
-    if (buf.block) cudaFree(buf.block);
-    if (buf.host) cudaFreeHost(buf.host);
-    buf = RenderBuffers{};
-}
+void ctx_give_render(sms_ctx *c, RenderBuffers &buf) { c->render_keep->give(buf); }
 
 void ctx_set_render_spp(sms_ctx *c, uint32_t spp) {
     if (c) c->render_spp = spp;
@@ -1378,7 +1343,7 @@ sms_status ctx_build_lean(sms_ctx *c) {
     if (total > 0xffffffffull) return fail(SMS_ERR_UNSUPPORTED, "slope map too large for the LEAN pyramid");
     CUDA_TRY(cudaSetDevice(c->device));
     void *p = nullptr;
-    CUDA_TRY(cudaMalloc(&p, total * sizeof(float)));
+    CUDA_TRY(device_malloc(&p, total * sizeof(float)));
     c->lean = reinterpret_cast<float *>(p);
     CUDA_TRY(launch_lean_build(c->dsc, c->lean, offs, levels, c->stream));
     c->dsc.lean = c->lean;

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/sms_gb300.h"
+#include "sms_keep.h"
 #include "sms_mlp.h"
 
 namespace sms {
@@ -158,17 +159,10 @@ sms_status ctx_glint_connect(sms_ctx *c, const float *q, uint32_t n, uint64_t se
                              const uint64_t *streams, sms_result *out);
 // Checks the glints scene, then builds the LEAN pyramid (ctx_build_lean).
 sms_status ctx_ensure_lean(sms_ctx *c);
-// Buffers of one render call, owned by the caller between take and give: a
-// device block of at least `bytes` and two words of pinned host memory.  The
-// context keeps the last given back (up to kRenderKeepBytes) for the next
-// render; several threads may take at once.
-struct RenderBuffers {
-    char *block = nullptr;
-    size_t bytes = 0;
-    uint32_t *host = nullptr;
-};
-cudaError_t ctx_take_render(sms_ctx *c, size_t bytes, RenderBuffers &out);
-void ctx_give_render(sms_ctx *c, RenderBuffers &buf);
+// Buffers of one render call (sms_keep.h): the context keeps the last given
+// back for the next render.
+cudaError_t ctx_take_render(sms_ctx *c, size_t bytes, sms::RenderBuffers &out);
+void ctx_give_render(sms_ctx *c, sms::RenderBuffers &buf);
 // Samples per pixel of the context's last render (sms_render_spp_done).
 void ctx_set_render_spp(sms_ctx *c, uint32_t spp);
 // Builds the LEAN pyramid of the scene's normal map on first use (the

@@ -95,7 +95,7 @@ sms_status ensure_act(sms_proposal *p, int batch, cudaStream_t s) {
         p->act_batch = 0;
     }
     const size_t hb = align256((size_t)mlp::kHRows * batch * 2), db = (size_t)mlp::kDzRows * batch * 2;
-    PTRY(cudaMalloc(&p->act, hb + db));
+    PTRY(device_malloc(&p->act, hb + db));
     p->act_batch = batch;
     p->net.hT = reinterpret_cast<__nv_bfloat16 *>(p->act);
     p->net.dzT = reinterpret_cast<__nv_bfloat16 *>(reinterpret_cast<char *>(p->act) + hb);
@@ -161,9 +161,9 @@ extern "C" sms_status sms_proposal_create(sms_ctx *ctx, int32_t caster, uint64_t
     const size_t total = off_mom + align256(2 * mlp::kIn * sizeof(double));
     sms_status st = SMS_OK;
     do {
-        cudaError_t e = cudaMalloc(&p->block, total);
+        cudaError_t e = device_malloc(&p->block, total);
         if (e != cudaSuccess) { st = cuda_fail(e, "cudaMalloc(proposal)"); break; }
-        e = cudaMalloc(&p->data, (size_t)mlp::kDataRows * capacity * sizeof(float));
+        e = device_malloc(reinterpret_cast<void **>(&p->data), (size_t)mlp::kDataRows * capacity * sizeof(float));
         if (e != cudaSuccess) { st = cuda_fail(e, "cudaMalloc(proposal training set)"); break; }
         char *b = reinterpret_cast<char *>(p->block);
         p->net.params = reinterpret_cast<float *>(b);
@@ -448,7 +448,7 @@ extern "C" sms_status sms_proposal_eval(sms_proposal *p, const float *feat, uint
     PTRY(cudaSetDevice(v.device));
     void *buf = nullptr;
     const size_t fb = (size_t)mlp::kIn * n * 4, ob = (size_t)mlp::kGmmParams * n * 4;
-    PTRY(cudaMalloc(&buf, fb + ob));
+    PTRY(device_malloc(&buf, fb + ob));
     float *df = reinterpret_cast<float *>(buf), *dout = reinterpret_cast<float *>(reinterpret_cast<char *>(buf) + fb);
     cudaError_t e = cudaMemcpyAsync(df, feat, fb, cudaMemcpyHostToDevice, v.stream);
     if (e == cudaSuccess) e = mlp::launch_forward(p->net, df, n, dout, mixture != 0, v.num_sms, v.stream);
