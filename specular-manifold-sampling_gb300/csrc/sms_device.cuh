@@ -104,9 +104,11 @@ SMS_HD f3 normalize(f3 a) { return a * (1.f / sqrtf(dot(a, a))); }
 #ifdef __CUDA_ARCH__
 SMS_HD float norm2_x(f3 a) { return __fmaf_rn(a.z, a.z, __fmaf_rn(a.x, a.x, __fmul_rn(a.y, a.y))); }
 SMS_HD float norm2_y(f3 a) { return __fmaf_rn(a.z, a.z, __fmaf_rn(a.y, a.y, __fmul_rn(a.x, a.x))); }
+SMS_HD float rounded_square(float a) { return __fmul_rn(a, a); }
 #else
 SMS_HD float norm2_x(f3 a) { return dot(a, a); }
 SMS_HD float norm2_y(f3 a) { return dot(a, a); }
+SMS_HD float rounded_square(float a) { return a * a; }
 #endif
 SMS_HD f3 normalize_x(f3 a) { return a * (1.f / sqrtf(norm2_x(a))); }
 SMS_HD f3 normalize_y(f3 a) { return a * (1.f / sqrtf(norm2_y(a))); }
@@ -315,12 +317,16 @@ struct Hit {
 // FP64, sphere.cpp:275-297).  The discriminant is formed from the vector to the
 // closest approach instead of b^2 - 4ac, which keeps FP32 accurate at the
 // distances of these scenes.  Same [mint, maxt] / inside-segment rules.
+// kRounded: the square of the radius is rounded before its two uses.  Otherwise
+// the compiler folds it into a difference or not by the code around, which
+// moves hit points by a last bit between two kernels.
+template <bool kRounded = false>
 SMS_HD bool sphere_hit(float4 s, f3 o, f3 d, float mint, float maxt, float &t_out) {
     f3 oc = o - mk(s.x, s.y, s.z);
     float a = dot(d, d);
     float b = dot(oc, d);                 // half of the reference's B
     f3 qv = oc - d * (b / a);
-    float r2 = s.w * s.w;
+    float r2 = kRounded ? rounded_square(s.w) : s.w * s.w;
     float disc = a * (r2 - dot(qv, qv));
     if (!(disc >= 0.f)) return false;
     float c = dot(oc, oc) - r2;
@@ -379,8 +385,9 @@ SMS_HD bool box2(float lox, float loy, float loz, float hix, float hiy, float hi
 // whole scene; one traversal loop serves both so that lanes of a warp casting
 // different kinds of rays still traverse together.  kTree: the launching
 // kernel holds the top sc.n_tnodes node records in shared memory (a separate
-// instantiation, so that kernels without it keep the plain fetch).  Returns false and sets *err on stack overflow (treated as miss).
-template <bool kTree = false>
+// instantiation, so that kernels without it keep the plain fetch); kRounded: see
+// sphere_hit.  Returns false and sets *err on stack overflow (treated as miss).
+template <bool kTree = false, bool kRounded = false>
 SMS_HD bool trace(const DevScene &sc, f3 o, f3 d, float mint, float maxt, bool any_hit, Hit &hit,
                   uint32_t &err) {
     hit.t = maxt; hit.shape = -1; hit.prim = 0; hit.u = hit.v = 0.f;
@@ -394,7 +401,7 @@ SMS_HD bool trace(const DevScene &sc, f3 o, f3 d, float mint, float maxt, bool a
     bool found = false;
     for (int i = 0; i < sc.n_spheres; ++i) {
         float t;
-        if (sphere_hit(sc.sphere[i], o, d, mint, hit.t, t) && (!found || t < hit.t)) {
+        if (sphere_hit<kRounded>(sc.sphere[i], o, d, mint, hit.t, t) && (!found || t < hit.t)) {
             hit.t = t; hit.shape = sc.sphere_shape[i]; found = true;
             if (any_hit) return true;
         }

@@ -603,6 +603,8 @@ SMS_D uint32_t bounce_path(const PtState &S, int depth, uint32_t slot, uint32_t 
 template <bool kMneeCheck, bool kFinish>
 __global__ void __launch_bounds__(kPtBlock, kBounceBlocks) pt_bounce_kernel(DevScene sc, PtParams P, PtState S, int depth,
                                                              uint32_t n, DevCounters *ctr, PtCam cam) {
+    // the bounce launches and the finishing one cast the same rays to the last bit
+    constexpr bool kRounded = !kMneeCheck;
     const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t i = bounce_path(S, depth, slot, n);
     int want = 0, alive_out = 0;
@@ -714,7 +716,7 @@ __global__ void __launch_bounds__(kPtBlock, kBounceBlocks) pt_bounce_kernel(DevS
                 float bw;
                 if (nm_conductor_sample(sc, s, n_sh, si.dp_du, uo, vo, wiw, bwo, bw)) {
                     Hit hb;
-                    trace(sc, si.p, bwo, kRayEps * (1.f + max_abs(si.p)), INFINITY, false, hb, err);
+                    trace<false, kRounded>(sc, si.p, bwo, kRayEps * (1.f + max_abs(si.p)), INFINITY, false, hb, err);
                     if (hb.shape >= 0 && sc.shapes[hb.shape].emitter >= 0) {
                         const DevShape &es = sc.shapes[hb.shape];
                         const f3 ep = si.p + bwo * hb.t;
@@ -788,7 +790,7 @@ __global__ void __launch_bounds__(kPtBlock, kBounceBlocks) pt_bounce_kernel(DevS
                 if (got) {
                     Hit hs;
                     float mint = kRayEps * (1.f + max_abs(si.p));
-                    bool occ = trace(sc, si.p, ds.d, mint, ds.dist * (1.f - kShadowEps), true, hs, err);
+                    bool occ = trace<false, kRounded>(sc, si.p, ds.d, mint, ds.dist * (1.f - kShadowEps), true, hs, err);
                     if (!occ && smooth) {
                         const f3 wo = mk(dot(ds.d, fs), dot(ds.d, ft), dot(ds.d, n_sh));
                         // the normalmap BSDF with uv partials evaluates its
@@ -853,7 +855,7 @@ __global__ void __launch_bounds__(kPtBlock, kBounceBlocks) pt_bounce_kernel(DevS
             } else {
                 f3 d2 = fs * bs.wo.x + ft * bs.wo.y + n_sh * bs.wo.z;
                 Hit h2;
-                trace(sc, si.p, d2, kRayEps * (1.f + max_abs(si.p)), INFINITY, false, h2, err);
+                trace<false, kRounded>(sc, si.p, d2, kRayEps * (1.f + max_abs(si.p)), INFINITY, false, h2, err);
                 if (filtered_ms) {
                     // PathRecord::state_transition (path_filtered_ms.cpp:244-300)
                     const bool nv = h2.shape >= 0;
