@@ -81,25 +81,45 @@ struct ChainOffsets {
     float *pdf = nullptr;         // first path: product of the offset densities
 };
 
+// How the code of a walk is written out, which decides what the compiler fuses
+// and so the last bits of the walk and of its contribution.  The walks between
+// wavy faces are chaotic: other last bits are other solutions and counts, so
+// each kernel keeps the form its results were first given with
+// (tests/test_gpu_chain_digests.py).
+//   kChainLoop      a loop over the vertices, one chain: the fast one
+//   kChainUnrolled  unrolled traces, the proposed chain beside the last one:
+//                   first walks of rough chains and of three vertices, whose
+//                   contributions round differently in a loop (three vertices,
+//                   20,011 points: 4.48 ms looped, 4.68)
+//   kChainPlain     as unrolled, no squared length written out, the last
+//                   iteration's ray cast: the per-walk entry point and the
+//                   MNEE test of the path tracer
+enum ChainForm { kChainLoop, kChainUnrolled, kChainPlain };
+template <int K, bool kRough>
+constexpr ChainForm first_walk_form() { return K == 3 || kRough ? kChainUnrolled : kChainLoop; }
+// Whether the vertex lengths of the angle-difference constraint are written out.
+template <int K, ChainForm kForm>
+constexpr bool pinned_lengths() { return K > 1 && kForm != kChainPlain; }
+
 // Trace a specular chain from x0 along wo, reflecting or refracting at each hit
 // (sample_seed_path :327-397, reproject :865-917).  tmpl (K shape ids) or
 // null; check_flags restricts hits to caster_multi / bouncer shapes; straight
 // keeps the direction at every hit (the MNEE seed path, :378-397).  kRough:
 // scattering about the offset normals of co (:380-382, :894-897).
-// The loop over the vertices stays a loop: one traversal per call site instead
-// of K.  Unrolled, the walk kernels of chains of two were so long that their
+// kChainLoop: the loop over the vertices stays a loop, one traversal per call
+// site instead of K.  Unrolled, the walk kernels of chains of two were so long that their
 // warps waited more for instructions (11 of 32 cycles an instruction) than for
 // memory: 65,536 slab points, biased, 36.4 -> 30.8 ms; 20,011 points, unbiased,
 // 3.42 -> 3.21 ms.  The chain then lies in local memory, which costs less.
 // Unrolling the constraint loop of chain_step pays (32.5 ms as a loop).
-template <int K, bool kNM = false, bool kRough = false>
+template <int K, bool kNM = false, bool kRough = false, ChainForm kForm = kChainLoop>
 SMS_D bool trace_chain(const DevScene &sc, f3 x0, f3 wo, const int *tmpl, bool check_flags, Chain<K> &c,
                        int *shapes, uint32_t &err, LaneStats &st, bool straight = false,
                        ChainOffsets<K> co = ChainOffsets<K>()) {
     f3 o = x0;
     float mint = kRayEps;
     if (kRough && co.draw) *co.pdf = 1.f;
-    #pragma unroll 1
+    #pragma unroll (kForm == kChainLoop ? 1 : K)
     for (int b = 0; b < K; ++b) {
         Hit h;
         trace(sc, o, wo, mint, INFINITY, false, h, err);
@@ -143,22 +163,29 @@ SMS_D bool trace_chain(const DevScene &sc, f3 x0, f3 wo, const int *tmpl, bool c
     return true;
 }
 
+template <ChainForm kForm>
+SMS_D f3 seed_direction(f3 to) { return kForm == kChainLoop ? normalize_y(to) : normalize(to); }
+template <ChainForm kForm>
+SMS_D f3 newton_direction(f3 to) { return kForm == kChainLoop ? normalize_x(to) : normalize(to); }
+
 // The seed path of a walk (sample_seed_path :280-408): toward the sampled
 // point x1, or with cfg.mnee_init along the straight line toward the MNEE
 // target without scattering.
-template <int K, bool kNM = false, bool kRough = false>
+template <int K, bool kNM = false, bool kRough = false, ChainForm kForm = kChainLoop>
 SMS_D bool seed_chain(const DevScene &sc, const SolverCfg &cfg, int caster, f3 x0, f3 x1, f3 lp, const int *tmpl,
                       Chain<K> &c, int *shapes, uint32_t &err, LaneStats &st,
                       ChainOffsets<K> co = ChainOffsets<K>()) {
     if (cfg.mnee_init)
-        return trace_chain<K, kNM, kRough>(sc, x0, normalize_y(mnee_target(sc.shapes[caster], lp) - x0), tmpl, true, c,
-                                           shapes, err, st, true, co);
-    return trace_chain<K, kNM, kRough>(sc, x0, normalize_y(x1 - x0), tmpl, true, c, shapes, err, st, false, co);
+        return trace_chain<K, kNM, kRough, kForm>(sc, x0, seed_direction<kForm>(mnee_target(sc.shapes[caster], lp) - x0),
+                                                  tmpl, true, c, shapes, err, st, true, co);
+    return trace_chain<K, kNM, kRough, kForm>(sc, x0, seed_direction<kForm>(x1 - x0), tmpl, true, c, shapes, err, st,
+                                              false, co);
 }
 
 // Angle-difference constraint of vertex i and its blocks w.r.t. the previous,
 // current and next vertex (:631-857); `no` is the vertex's offset normal in
 // its shading frame (:707-717; (0, 0, 1) keeps the vertex normal).
+template <bool kPinned>
 SMS_D bool vertex_anglediff(f3 xp, const Vtx &vc, f3 xn, const Vtx *vp, const Vtx *vn, float &c0, float &c1,
                             M2 &prev, M2 &cur, M2 &next, f3 no = f3{0.f, 0.f, 1.f}) {
     prev = {0.f, 0.f, 0.f, 0.f};
@@ -166,13 +193,13 @@ SMS_D bool vertex_anglediff(f3 xp, const Vtx &vc, f3 xn, const Vtx *vp, const Vt
     next = prev;
     c0 = c1 = 0.f;
     f3 wo = xn - vc.p;
-    float ilo = sqrtf(norm2_x(wo));
+    float ilo = kPinned ? sqrtf(norm2_x(wo)) : length(wo);
     if (ilo < 1e-3f) return false;
     ilo = 1.f / ilo; wo = wo * ilo;
     f3 dwo_du = (vc.dp_du - wo * dot(wo, vc.dp_du)) * -ilo;
     f3 dwo_dv = (vc.dp_dv - wo * dot(wo, vc.dp_dv)) * -ilo;
     f3 wi = xp - vc.p;
-    float ili = sqrtf(norm2_x(wi));
+    float ili = kPinned ? sqrtf(norm2_x(wi)) : length(wi);
     if (ili < 1e-3f) return false;
     ili = 1.f / ili; wi = wi * ili;
     f3 dwi_du = (vc.dp_du - wi * dot(wi, vc.dp_du)) * -ili;
@@ -304,7 +331,7 @@ SMS_D bool vertex_halfvector(f3 xp, const Vtx &vc, f3 xn, const Vtx *vp, const V
 // Constraints, blocks and the block-Thomas Newton step (:1192-1232).  Returns
 // false when a constraint or the solve fails; conv = all |C_i| <= threshold;
 // dx0 = step of the first vertex (the only one reprojection uses).
-template <int K, bool kRough = false>
+template <int K, bool kRough, bool kPinned>
 SMS_D bool chain_step(const SolverCfg &cfg, f3 x0, f3 lp, const Chain<K> &c, bool &conv, float &dx0u, float &dx0v,
                       const f3 *offs = nullptr) {
     float C0[K], C1[K];
@@ -317,7 +344,7 @@ SMS_D bool chain_step(const SolverCfg &cfg, f3 x0, f3 lp, const Chain<K> &c, boo
         const Vtx *vn = i < K - 1 ? &c.v[i + 1] : nullptr;
         const f3 no = kRough && offs ? offs[i] : f3{0.f, 0.f, 1.f};
         bool ok = cfg.halfvector ? vertex_halfvector(xp, c.v[i], xn, vp, vn, C0[i], C1[i], P[i], Cu[i], N[i], no)
-                                 : vertex_anglediff(xp, c.v[i], xn, vp, vn, C0[i], C1[i], P[i], Cu[i], N[i], no);
+                                 : vertex_anglediff<kPinned>(xp, c.v[i], xn, vp, vn, C0[i], C1[i], P[i], Cu[i], N[i], no);
         if (!ok) return false;
     }
     M2 tmp[K], il[K];
@@ -359,7 +386,7 @@ SMS_D bool chain_step(const SolverCfg &cfg, f3 x0, f3 lp, const Chain<K> &c, boo
 
 // newton_solver (:410-498).  c holds the seed path on entry and the solution
 // on success; tmpl = the estimate's template shapes.
-template <int K, bool kNM = false, bool kRough = false>
+template <int K, bool kNM = false, bool kRough = false, ChainForm kForm = kChainLoop>
 SMS_D bool chain_newton(const DevScene &sc, const SolverCfg &cfg, f3 x0, f3 lp, const int *tmpl, Chain<K> &c,
                         int &it, uint32_t &err, LaneStats &st, const f3 *offs = nullptr) {
     ChainOffsets<K> co;
@@ -367,21 +394,35 @@ SMS_D bool chain_newton(const DevScene &sc, const SolverCfg &cfg, f3 x0, f3 lp, 
     it = 0;
     float beta = 1.f;
     bool need = true, conv = false, ok = true;
-    // first vertex of the last complete chain and the full Newton step from it
+    constexpr bool kPinned = pinned_lengths<K, kForm>();
+    float du = 0.f, dv = 0.f;
+    // kChainLoop: first vertex of the last complete chain and the full Newton step from it
     f3 vp = splat(0.f), step = vp;
     while (it < cfg.max_iterations) {
         if (need) {
-            float du = 0.f, dv = 0.f;
-            ok = chain_step<K, kRough>(cfg, x0, lp, c, conv, du, dv, offs);
-            vp = c.v[0].p;
-            step = c.v[0].dp_du * du + c.v[0].dp_dv * dv;
+            ok = chain_step<K, kRough, kPinned>(cfg, x0, lp, c, conv, du, dv, offs);
+            if constexpr (kForm == kChainLoop) {
+                vp = c.v[0].p;
+                step = c.v[0].dp_du * du + c.v[0].dp_dv * dv;
+            }
         }
         if (!ok) break;
         if (conv) break;
         // the last iteration's chain would be one no step is taken from
-        if (it + 1 >= cfg.max_iterations) { it++; break; }
-        const f3 p0 = vp - step * (cfg.step_scale * beta);
-        need = trace_chain<K, kNM, kRough>(sc, x0, normalize_x(p0 - x0), tmpl, false, c, nullptr, err, st, false, co);
+        if (kForm != kChainPlain && it + 1 >= cfg.max_iterations) { it++; break; }
+        if constexpr (kForm == kChainLoop) {
+            // the proposed chain replaces the last one: what a further step from
+            // that one needs is in vp and step
+            const f3 p0 = vp - step * (cfg.step_scale * beta);
+            need = trace_chain<K, kNM, kRough>(sc, x0, newton_direction<kForm>(p0 - x0), tmpl, false, c, nullptr, err,
+                                               st, false, co);
+        } else {
+            const f3 p0 = c.v[0].p - (c.v[0].dp_du * du + c.v[0].dp_dv * dv) * (cfg.step_scale * beta);
+            Chain<K> prop;
+            need = trace_chain<K, kNM, kRough, kForm>(sc, x0, newton_direction<kForm>(p0 - x0), tmpl, false, prop,
+                                                      nullptr, err, st, false, co);
+            if (need) c = prop;
+        }
         beta = need ? fminf(1.f, 2.f * beta) : 0.5f * beta;
         it++;
     }
@@ -408,6 +449,12 @@ SMS_D bool chain_admissible(f3 x0, f3 lp, const Chain<K> &c) {
         if ((c.v[i].eta == 1.f) ? refraction : !refraction) return false;
     }
     return true;
+}
+
+// dp_du du + dp_dv dv, the second product fused (chains of one vertex; see ChainForm).
+SMS_D f3 step_y(const Vtx &v, float du, float dv) {
+    return mk(__fmaf_rn(v.dp_dv.x, dv, __fmul_rn(v.dp_du.x, du)), __fmaf_rn(v.dp_dv.y, dv, __fmul_rn(v.dp_du.y, du)),
+              __fmaf_rn(v.dp_dv.z, dv, __fmul_rn(v.dp_du.z, du)));
 }
 
 // One lane's walk in chain_run: its seed path and Newton iterations, each one
@@ -468,13 +515,13 @@ SMS_D void chain_run(const DevScene &sc, const SolverCfg &cfg, int lanes, uint32
                 bool conv = false;
                 float du = 0.f, dv = 0.f;
                 go = w.it < cfg.max_iterations &&
-                     chain_step<K, kRough>(cfg, w.x0, w.lp, w.c, conv, du, dv, kRough ? w.offs : nullptr);
+                     chain_step<K, kRough, pinned_lengths<K, kChainLoop>()>(cfg, w.x0, w.lp, w.c, conv, du, dv, kRough ? w.offs : nullptr);
                 if (go && conv) {
                     w.ok = chain_admissible<K>(w.x0, w.lp, w.c);
                     go = false;
                 }
                 w.vp = w.c.v[0].p;
-                w.step = w.c.v[0].dp_du * du + w.c.v[0].dp_dv * dv;
+                w.step = K == 1 ? step_y(w.c.v[0], du, dv) : w.c.v[0].dp_du * du + w.c.v[0].dp_dv * dv;
             } else {
                 go = !w.seed;
                 w.beta = 0.5f * w.beta;
@@ -627,8 +674,8 @@ __global__ void __launch_bounds__(128) ms_walk_kernel(DevScene sc, SolverCfg cfg
         Chain<K> c;
         int shapes[K];
         int it = 0;
-        bool seed_ok = seed_chain<K, kNM>(sc, cfg, caster, x, x1, lp, nullptr, c, shapes, err, st);
-        bool ok = seed_ok && chain_newton<K, kNM>(sc, cfg, x, lp, shapes, c, it, err, st);
+        bool seed_ok = seed_chain<K, kNM, false, kChainPlain>(sc, cfg, caster, x, x1, lp, nullptr, c, shapes, err, st);
+        bool ok = seed_ok && chain_newton<K, kNM, false, kChainPlain>(sc, cfg, x, lp, shapes, c, it, err, st);
         float res[kMsWalkOutFields] = {ok ? 1.f : 0.f, (float)it, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, seed_ok ? 1.f : 0.f};
         if (ok) {
             res[2] = c.v[0].p.x; res[3] = c.v[0].p.y; res[4] = c.v[0].p.z;
@@ -666,8 +713,8 @@ __global__ void __launch_bounds__(128) ms_mnee_check_kernel(DevScene sc, SolverC
         Chain<K> c;
         int shapes[K];
         int it = 0;
-        bool ok = seed_chain<K, kNM>(sc, cfg, caster, x0, lp, lp, nullptr, c, shapes, err, st) &&
-                  chain_newton<K, kNM>(sc, cfg, x0, lp, shapes, c, it, err, st);
+        bool ok = seed_chain<K, kNM, false, kChainPlain>(sc, cfg, caster, x0, lp, lp, nullptr, c, shapes, err, st) &&
+                  chain_newton<K, kNM, false, kChainPlain>(sc, cfg, x0, lp, shapes, c, it, err, st);
         #pragma unroll
         for (int k = 0; k < K; ++k)
             if (ok && !(length(c.v[k].p - mk(R(4 + 3 * k), R(5 + 3 * k), R(6 + 3 * k))) < 1e-5f)) ok = false;
@@ -938,8 +985,11 @@ __global__ void __launch_bounds__(128) ms_first_kernel(DevScene sc, SolverCfg cf
                 for (int j = 0; j < 2 * K; ++j) dr[j] = rng.next_f32();
                 co.draw = dr; co.out = own; co.pdf = &own_pdf;
             }
-            bool ok = seed_chain<K, kNM, kRough>(sc, cfg, caster, Q.x, x1, L.p, nullptr, c, shapes, err, st, co) &&
-                      chain_newton<K, kNM, kRough>(sc, cfg, Q.x, L.p, shapes, c, it, err, st, kRough ? own : nullptr);
+            constexpr ChainForm kForm = first_walk_form<K, kRough>();
+            bool ok = seed_chain<K, kNM, kRough, kForm>(sc, cfg, caster, Q.x, x1, L.p, nullptr, c, shapes, err, st,
+                                                        co) &&
+                      chain_newton<K, kNM, kRough, kForm>(sc, cfg, Q.x, L.p, shapes, c, it, err, st,
+                                                          kRough ? own : nullptr);
             st.walks++;
             st.newton += (unsigned)it;
             nw++;
