@@ -433,7 +433,7 @@ def learned_study(torch, sms, W, ctx, dev, pairs=4 << 20, steps=20000, batch=819
     stream = torch.cuda.ExternalStream(ctx.stream, device=dev)
     cfg = W.water_config()
     ctx.set_config(cfg)
-    ctx.set_trial_group(0)   # 32 lanes per query for uniform seeds, 8 for learned ones
+    ctx.set_trial_group(0)
     prop = sms.SeedProposal(ctx, 0, seed=1, capacity=pairs)
     prop.set_options(sigma_scale, weighted)
     chunk = 1 << 20
@@ -461,7 +461,7 @@ def learned_study(torch, sms, W, ctx, dev, pairs=4 << 20, steps=20000, batch=819
     pix = W.plane_queries(np.stack([xx.ravel(), yy.ravel()], axis=1).astype(np.float32))
     npix = pix.shape[1]
 
-    # trial-group size for learned seeds, tuned on a 16-spp sample of the image
+    # launch shape for learned seeds, timed on a 16-spp sample of the image
     from sms_gb300.autotune import autotune_ss
     ctx.set_proposal(prop, 0.1)
     qs = torch.from_numpy(np.tile(pix, (1, 16))).to(f"cuda:{dev}")
@@ -471,7 +471,7 @@ def learned_study(torch, sms, W, ctx, dev, pairs=4 << 20, steps=20000, batch=819
     ws = torch.empty(ns, dtype=torch.int32, device=f"cuda:{dev}")
     torch.cuda.synchronize()
     tune = autotune_ss(sms, ctx, qs.data_ptr(), ns, vs.data_ptr(), cs.data_ptr(), ws.data_ptr(),
-                       blocks_per_sm=(0,), trial_groups=(8, 16, 32), treelets=(0,), chunks=(1,), seed=99)
+                       blocks_per_sm=(0,), trial_groups=(32,), treelets=(0,), chunks=(1,), seed=99)
     learned_group = tune["best"][1]
     ctx.set_proposal(None)
     ctx.set_launch(0, 0)

@@ -216,10 +216,9 @@ void      *sms_ctx_stream(sms_ctx *ctx);
 /* Launch shape of the persistent kernels: blocks per SM and threads per block
  * (0 = library default).  Set by the autotuner. */
 sms_status sms_ctx_set_launch(sms_ctx *ctx, int32_t blocks_per_sm, int32_t threads_per_block);
-/* Lanes of a warp of the single-scatter Bernoulli-trial kernel that take
- * trials, one each: 8, 16 or 32 (0 = 32).  Fewer lanes wait less for each
- * other and use less of the machine; results do not depend on it.  No
- * counterpart in the reference (a tuning knob of the batched solver). */
+/* Trial group: 0, 8, 16 or 32, others are refused.  Without effect: the trials
+ * of a query no longer share a group of lanes, and all lanes of a warp take
+ * trials.  No counterpart in the reference. */
 sms_status sms_ctx_set_trial_group(sms_ctx *ctx, int32_t group);
 /* Top node records of the scene's tree (stored breadth first) that the
  * Bernoulli-trial kernel copies into each block's shared memory before it
@@ -227,8 +226,8 @@ sms_status sms_ctx_set_trial_group(sms_ctx *ctx, int32_t group);
  * L1 for the top levels; results do not depend on it.  No counterpart in the
  * reference (a staging knob of the batched solver, set by the autotuner). */
 sms_status sms_ctx_set_treelet(sms_ctx *ctx, int32_t nodes);
-/* Rounds of trials a warp of the Bernoulli-trial kernel claims from the stream
- * of trials per atomic, at least; 1..64 (default 1).  Results do not depend on
+/* Rounds of trials a warp of the single-scatter Bernoulli-trial kernel claims
+ * from the stream of trials per atomic, at least; 1..64 (default 1).  Results do not depend on
  * it.  No counterpart in the reference (a tuning knob of the batched solver,
  * set by the autotuner). */
 sms_status sms_ctx_set_queue_chunk(sms_ctx *ctx, int32_t chunk);
@@ -548,7 +547,8 @@ sms_status sms_ctx_set_proposal(sms_ctx *ctx, sms_proposal *p, float defensive);
  * bounce Russian roulette (1, past rr_depth), emitter sampling (2, when it
  * runs) and BSDF sampling (1 + 2).  The SMS call at bounce `depth` of path p
  * draws from stream p + depth * 2^48 of state seed sms_render_sms_seed(seed).
- * Images therefore do not depend on the wavefront size. */
+ * Images therefore do not depend on the wavefront size, but for the order in
+ * which the samples of a pixel are summed. */
 typedef struct sms_camera {
     float   to_world[16];   /* row-major camera-to-world; camera space has x
                                left, y up, z forward (the reference's look_at) */

@@ -429,7 +429,8 @@ class Context:
         _check(_LIB.sms_ctx_set_launch(self._h, blocks_per_sm, threads_per_block))
 
     def set_trial_group(self, group: int = 0):
-        """Lanes per query of the Bernoulli-trial kernel (0 auto, 8, 16, 32)."""
+        """0, 8, 16 or 32; without effect (the trials of a query no longer
+        share a group of lanes)."""
         _check(_LIB.sms_ctx_set_trial_group(self._h, group))
 
     def set_treelet(self, nodes: int = 0):
@@ -438,7 +439,8 @@ class Context:
         _check(_LIB.sms_ctx_set_treelet(self._h, nodes))
 
     def set_queue_chunk(self, chunk: int = 1):
-        """Queries a Bernoulli-trial lane group claims per atomic (1..64)."""
+        """Rounds of trials a warp of the single-scatter Bernoulli-trial kernel
+        claims per atomic, at least (1..64)."""
         _check(_LIB.sms_ctx_set_queue_chunk(self._h, chunk))
 
     def stats(self) -> dict:

@@ -1,11 +1,11 @@
 """Launch-shape autotuner of the SMS solvers.
 
 Picks, for one context and a representative device-resident query sample,
-the persistent kernels' blocks per SM (warps per SM = 4 x blocks), the lanes
-of a warp of the Bernoulli-trial kernel that take trials (trial group), the
-number of top tree nodes the trial kernel stages in shared memory, and the
+the persistent kernels' blocks per SM (warps per SM = 4 x blocks), the number
+of top tree nodes the Bernoulli-trial kernel stages in shared memory, and the
 rounds of trials a warp claims from the stream per atomic (queue chunk); for
-the multi-scatter and glint estimators, blocks per SM.  The library's own
+the multi-scatter and glint estimators, blocks per SM.  The trial group is
+tried where a caller asks for it; it has no effect.  The library's own
 blocks per SM (0), which differ from kernel to kernel, are among the
 candidates.  Each candidate is timed with the library's own CUDA-event phase
 profile (sms_profile_read).  No candidate changes a result: the random
@@ -30,7 +30,7 @@ def _time_ss(ss, ctx, args, seed, repeats):
 
 
 def autotune_ss(sms, ctx, queries_ptr: int, n: int, value_ptr: int, count_ptr: int, walks_ptr: int,
-                blocks_per_sm=(0, 2, 4, 6, 8, 12, 16), trial_groups=(8, 16, 32), treelets=(0, 64, 128, 256, 384),
+                blocks_per_sm=(0, 2, 4, 6, 8, 12, 16), trial_groups=(32,), treelets=(0, 64, 128, 256, 384),
                 chunks=(1, 2, 4), seed: int = 12345, repeats: int = 2) -> dict:
     """Time every (blocks_per_sm, trial_group) pair on the sample (device
     pointers, as SpecularManifoldSingleScatter.specular_manifold_sampling_device),

@@ -487,9 +487,8 @@ struct sms_ctx {
     int num_sms = 0;
     int blocks_per_sm = 0;
     int threads = 128;
-    int trial_group = 0;          // lanes per query of the Bernoulli-trial kernel (0: auto)
     uint32_t treelet = 0;         // node records the trial kernel stages in shared memory
-    int queue_chunk = 1;          // queries a trial-kernel lane group claims per atomic
+    int queue_chunk = 1;          // rounds of trials a single-scatter trial warp claims per atomic, at least
     // device staging for the host-pointer entry points
     void *io = nullptr;
     size_t io_bytes = 0;
@@ -829,7 +828,6 @@ extern "C" sms_status sms_ctx_set_trial_group(sms_ctx *c, int32_t group) {
     if (!c) return fail(SMS_ERR_INVALID_ARG, "null context");
     if (group != 0 && group != 8 && group != 16 && group != 32)
         return fail(SMS_ERR_INVALID_ARG, "trial group must be 0 (auto), 8, 16 or 32");
-    c->trial_group = group;
     return SMS_OK;
 }
 
@@ -1023,7 +1021,7 @@ sms_status ctx_ss_connect(sms_ctx *c, const float *q, uint32_t n, uint64_t seed,
     sc.queue_chunk = c->queue_chunk;
     CUDA_TRY(launch_ss_connect(c->dsc, sc, q, n, seed, stream_off, out->value, out->count, out->walks, c->ctr, scr,
                                c->num_sms, c->blocks_per_sm, &c->timer, c->stream, c->prop ? &pr : nullptr,
-                               c->trial_group, c->treelet));
+                               c->treelet));
     return SMS_OK;
 }
 
@@ -1160,7 +1158,6 @@ bool ctx_view(sms_ctx *c, CtxView &out) {
     out.frames = c->frames.data();
     out.n_shapes = (int)c->frames.size();
     out.proposal_bound = c->prop != nullptr;
-    out.trial_group = c->trial_group;
     out.bounces = c->cfg.bounces;
     out.bsdf_strategy_only = c->cfg.bsdf_strategy_only;
     out.nm_rough = c->nm_rough;

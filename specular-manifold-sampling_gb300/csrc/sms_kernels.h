@@ -78,7 +78,7 @@ cudaError_t launch_ss_connect(const DevScene &sc, const SolverCfg &cfg, const fl
                               uint64_t seed, uint64_t stream_off, float *value, int *count, int *walks,
                               DevCounters *ctr, const SsScratch &scr, int num_sms, int blocks_per_sm,
                               PhaseTimer *tm, cudaStream_t s, const mlp::SeedProposal *prop = nullptr,
-                              int trial_group = 0, uint32_t treelet = 0);
+                              uint32_t treelet = 0);
 // The proposal network for every query of a batch (ss_proposal_kernel).
 cudaError_t launch_ss_proposal(const DevScene &sc, const SolverCfg &cfg, const float *q, uint32_t n, uint64_t seed,
                                uint64_t stream_off, const mlp::SeedProposal &pr, int num_sms, cudaStream_t s);
@@ -93,7 +93,7 @@ cudaError_t launch_ss_biased_nm(int var, const DevScene &sc, const SolverCfg &cf
 cudaError_t launch_ss_caster_nm(int var, const DevScene &sc, const SolverCfg &cfg, int c, const float *q, uint32_t n,
                                 uint64_t seed, uint64_t stream_off, float *value, int *count, int *walks,
                                 DevCounters *ctr, const SsScratch &scr, int num_sms, int bps, PhaseTimer *tm,
-                                cudaStream_t s, int trial_group);
+                                cudaStream_t s);
 // Training pairs for a learned proposal (see ss_collect_kernel).
 cudaError_t launch_ss_collect(const DevScene &sc, const SolverCfg &cfg, int caster, const float *q, uint32_t n,
                               uint64_t seed, uint64_t stream_off, int per_query, const mlp::SeedFrame &fr,
@@ -129,7 +129,6 @@ struct CtxView {
     const mlp::SeedFrame *frames;   // learned-proposal uv frame per shape
     int n_shapes;
     bool proposal_bound;            // a learned proposal seeds the SS estimator
-    int trial_group;                // lanes per query of the trial kernel (0: auto)
     int bounces;                    // multi-scatter chain length (sms_config::bounces)
     int bsdf_strategy_only, sms_strategy_only;   // glints MIS switches (sms_config)
     bool nm_rough;                  // the normal-mapped shape is rough (alpha > 0)

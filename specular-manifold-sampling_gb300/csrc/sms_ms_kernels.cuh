@@ -88,15 +88,15 @@ struct ChainOffsets {
 // (tests/test_gpu_chain_digests.py).
 //   kChainLoop      a loop over the vertices, one chain: the fast one
 //   kChainUnrolled  unrolled traces, the proposed chain beside the last one:
-//                   first walks of rough chains and of three vertices, whose
-//                   contributions round differently in a loop (three vertices,
-//                   20,011 points: 4.48 ms looped, 4.68)
+//                   first walks of rough chains (but for three vertices) and
+//                   smooth ones of three, which round differently in a loop
+//                   (smooth, 20,011 points: 4.48 ms looped, 4.68)
 //   kChainPlain     as unrolled, no squared length written out, the last
 //                   iteration's ray cast: the per-walk entry point and the
 //                   MNEE test of the path tracer
 enum ChainForm { kChainLoop, kChainUnrolled, kChainPlain };
 template <int K, bool kRough>
-constexpr ChainForm first_walk_form() { return K == 3 || kRough ? kChainUnrolled : kChainLoop; }
+constexpr ChainForm first_walk_form() { return kRough != (K == 3) ? kChainUnrolled : kChainLoop; }
 // Whether the vertex lengths of the angle-difference constraint are written out.
 template <int K, ChainForm kForm>
 constexpr bool pinned_lengths() { return K > 1 && kForm != kChainPlain; }
@@ -1042,9 +1042,9 @@ template <int K, bool kNM, bool kRough = false>
 __global__ void __launch_bounds__(128, kMsWalkBlocks)
 ms_trials_kernel(DevScene sc, SolverCfg cfg, int ci, const float *__restrict__ qs, uint32_t n, uint64_t seed,
                  uint64_t stream_off, int *__restrict__ count, SsScratch scr, const int *__restrict__ tmpl_in,
-                 DevCounters *ctr, int pass) {
+                 DevCounters *ctr, int pass, TrialRule rule) {
     const int cap = cfg.max_trials > 0 ? cfg.max_trials : kTrialHardLimit;
-    TrialStream ts(*(volatile unsigned *)&ctr->trial_count, cap, pass);
+    TrialStream ts(*(volatile unsigned *)&ctr->trial_count, cap, pass, 32, rule);
     if (ts.total == 0) return;
     __shared__ TrialBuffer bufs[4];
     TrialBuffer &buf = bufs[threadIdx.x >> 5];
@@ -1055,7 +1055,7 @@ ms_trials_kernel(DevScene sc, SolverCfg cfg, int ci, const float *__restrict__ q
     uint32_t qi = 0;
     int t = 0;
     auto start = [&](int want, int rank, ChainWalk<K> &w) {
-        if (!ts.next(buf, scr.list, count, ctr, pass, cfg.queue_chunk, want, rank, qi, t)) return false;
+        if (!ts.next(buf, scr.list, count, ctr, pass, 1, want, rank, qi, t)) return false;
         const Query Q = load_query(qs, n, qi);
         Pcg32 rng = query_rng(seed, query_stream(cfg, stream_off, qi), 0);
         Light L;
@@ -1136,8 +1136,10 @@ cudaError_t ms_connect_k(const DevScene &sc, const SolverCfg &cfg, const float *
         first<<<first_walk_blocks(n, lanes), 128, 0, s>>>(sc, cfg, c, q, n, seed, stream_off, value, count, walks, scr, tmpl, ctr, lanes);
         const int tblocks = num_sms * (bps > 0 ? bps : kMsWalkBlocks);
         const int cap = cfg.max_trials > 0 ? cfg.max_trials : kTrialHardLimit;
-        for (int pass = trial_split_possible(n, cap, tblocks) ? 0 : 1; pass < 2; ++pass)
-            trials<<<tblocks, 128, 0, s>>>(sc, cfg, c, q, n, seed, stream_off, count, scr, tmpl, ctr, pass);
+        TrialRule rule;
+        rule.split = cfg.mnee_init ? kSplitAlways : kSplitLong;
+        for (int pass = trial_split_possible(rule, n, cap, tblocks) ? 0 : 1; pass < 2; ++pass)
+            trials<<<tblocks, 128, 0, s>>>(sc, cfg, c, q, n, seed, stream_off, count, scr, tmpl, ctr, pass, rule);
         // result += value / m_offset_normals_pdf (:198)
         const float *pdf = kRough ? reinterpret_cast<const float *>(tmpl + (size_t)kMaxBounces * n) +
                                         (size_t)(3 * kMaxBounces) * n : nullptr;

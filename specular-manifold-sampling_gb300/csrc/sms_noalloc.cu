@@ -142,8 +142,7 @@ extern "C" sms_status sms_ss_connect_batch_noalloc(sms_ctx *ctx, const float *qu
     // No phase timer: recording it may create CUDA events (an allocation), so
     // these calls do not appear in sms_profile_read.
     e = launch_ss_connect(*v.scene, v.solver, queries_dev, n, seed, stream_offset, out_dev->value, out_dev->count,
-                          out_dev->walks, v.counters, scr, v.num_sms, v.blocks_per_sm, nullptr, v.stream, nullptr,
-                          v.trial_group);
+                          out_dev->walks, v.counters, scr, v.num_sms, v.blocks_per_sm, nullptr, v.stream, nullptr);
     if (e != cudaSuccess) return set_last_error(SMS_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
     return SMS_OK;
 }

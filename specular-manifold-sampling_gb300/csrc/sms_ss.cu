@@ -246,7 +246,7 @@ static int ss_variant(const DevScene &sc, const SolverCfg &cfg, int c) {
 cudaError_t launch_ss_connect(const DevScene &sc, const SolverCfg &cfg, const float *q, uint32_t n, uint64_t seed,
                               uint64_t stream_off, float *value, int *count, int *walks, DevCounters *ctr,
                               const SsScratch &scr, int num_sms, int blocks_per_sm, PhaseTimer *tm,
-                              cudaStream_t s, const mlp::SeedProposal *prop, int trial_group, uint32_t treelet) {
+                              cudaStream_t s, const mlp::SeedProposal *prop, uint32_t treelet) {
     if (n == 0) return cudaSuccess;
     const int bps = blocks_per_sm > 0 ? blocks_per_sm : 16;
     if (cfg.biased) {
@@ -271,13 +271,13 @@ cudaError_t launch_ss_connect(const DevScene &sc, const SolverCfg &cfg, const fl
         const int var = ss_variant(sc, cfg, c);
         if (var & 4)
             e = launch_ss_caster_nm(var, sc, cfg, c, q, n, seed, stream_off, value, count, walks, ctr, scr, num_sms,
-                                    blocks_per_sm, tm, s, trial_group);
+                                    blocks_per_sm, tm, s);
         else if (var)
             e = ss_caster_launch<1, true>(sc, cfg, c, q, n, seed, stream_off, value, count, walks, ctr, scr, num_sms,
-                                          blocks_per_sm, tm, s, prop, trial_group, treelet);
+                                          blocks_per_sm, tm, s, prop, treelet);
         else
             e = ss_caster_launch<0, true>(sc, cfg, c, q, n, seed, stream_off, value, count, walks, ctr, scr, num_sms,
-                                          blocks_per_sm, tm, s, prop, trial_group, treelet);
+                                          blocks_per_sm, tm, s, prop, treelet);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;

@@ -287,10 +287,10 @@ template <bool kLearned, int kVar, bool kTree = false>
 __global__ void __launch_bounds__(128, ss_walk_blocks(kVar)) ss_trials_kernel(DevScene sc, SolverCfg cfg, int c, const float *__restrict__ qs,
                                                         uint32_t n, uint64_t seed, uint64_t stream_off,
                                                         int *__restrict__ count, SsScratch scr, DevCounters *ctr,
-                                                        mlp::SeedProposal pr, int pass, int lanes) {
+                                                        mlp::SeedProposal pr, int pass, TrialRule rule) {
     constexpr bool kRough = (kVar & 1) != 0, kTwo = (kVar & 2) != 0, kNM = (kVar & 4) != 0;
     const int cap = cfg.max_trials > 0 ? cfg.max_trials : kTrialHardLimit;
-    TrialStream ts(*(volatile unsigned *)&ctr->trial_count, cap, pass, lanes);
+    TrialStream ts(*(volatile unsigned *)&ctr->trial_count, cap, pass, 32, rule);
     if (ts.total == 0) return;
     if (kTree) tree_smem_fill(sc);
     __shared__ TrialBuffer bufs[4];
@@ -369,7 +369,7 @@ template <int kVar, bool kLearnedOk>
 cudaError_t ss_caster_launch(const DevScene &sc, const SolverCfg &cfg, int c, const float *q, uint32_t n,
                              uint64_t seed, uint64_t stream_off, float *value, int *count, int *walks,
                              DevCounters *ctr, const SsScratch &scr, int num_sms, int bps, PhaseTimer *tm,
-                             cudaStream_t s, const mlp::SeedProposal *prop, int trial_group, uint32_t treelet = 0) {
+                             cudaStream_t s, const mlp::SeedProposal *prop, uint32_t treelet = 0) {
     const bool learned = kLearnedOk && prop && prop->shape == sc.casters_ss[c];
     // the trial kernel holds the top `treelet` node records in shared memory
     // (plain and rough casters)
@@ -408,9 +408,13 @@ cudaError_t ss_caster_launch(const DevScene &sc, const SolverCfg &cfg, int c, co
     }
     const int tblocks = num_sms * (bps > 0 ? bps : ss_walk_blocks(kVar));
     const int cap = cfg.max_trials > 0 ? cfg.max_trials : kTrialHardLimit;
-    for (int pass = trial_split_possible(n, cap, tblocks) ? 0 : 1; pass < 2; ++pass)
-        trials<<<tblocks, 128, tsmem, s>>>(st, cfg, c, q, n, seed, stream_off, count, scr, ctr, pr, pass,
-                                           trial_group > 0 ? trial_group : 32);
+    TrialRule rule;
+    rule.split = cfg.mnee_init ? kSplitAlways : (kVar & 2) ? kSplitLong : kSplitNever;
+    rule.claim_by_row = true;
+    rule.warps = sc.n_tris <= kSmallTree ? kSmallTreeWarps * num_sms : 0;
+    rule.even_end = true;
+    for (int pass = trial_split_possible(rule, n, cap, tblocks) ? 0 : 1; pass < 2; ++pass)
+        trials<<<tblocks, 128, tsmem, s>>>(st, cfg, c, q, n, seed, stream_off, count, scr, ctr, pr, pass, rule);
     const uint32_t stride = (learned ? 3u : 2u) + ((kVar & 2) ? 2u : 0u);
     trials_finish_kernel<<<finish_blocks(n, num_sms), 128, 0, s>>>(n, value, count, walks, scr, nullptr, cap,
                                                                    cfg.max_trials <= 0, stride, kPhaseSsTrials, ctr);

@@ -19,20 +19,20 @@ cudaError_t launch_ss_biased_nm(int var, const DevScene &sc, const SolverCfg &cf
 cudaError_t launch_ss_caster_nm(int var, const DevScene &sc, const SolverCfg &cfg, int c, const float *q, uint32_t n,
                                 uint64_t seed, uint64_t stream_off, float *value, int *count, int *walks,
                                 DevCounters *ctr, const SsScratch &scr, int num_sms, int bps, PhaseTimer *tm,
-                                cudaStream_t s, int trial_group) {
+                                cudaStream_t s) {
     switch (var) {
         case 4:
             return ss_caster_launch<4, false>(sc, cfg, c, q, n, seed, stream_off, value, count, walks, ctr, scr,
-                                              num_sms, bps, tm, s, nullptr, trial_group);
+                                              num_sms, bps, tm, s, nullptr);
         case 5:
             return ss_caster_launch<5, false>(sc, cfg, c, q, n, seed, stream_off, value, count, walks, ctr, scr,
-                                              num_sms, bps, tm, s, nullptr, trial_group);
+                                              num_sms, bps, tm, s, nullptr);
         case 6:
             return ss_caster_launch<6, false>(sc, cfg, c, q, n, seed, stream_off, value, count, walks, ctr, scr,
-                                              num_sms, bps, tm, s, nullptr, trial_group);
+                                              num_sms, bps, tm, s, nullptr);
         default:
             return ss_caster_launch<7, false>(sc, cfg, c, q, n, seed, stream_off, value, count, walks, ctr, scr,
-                                              num_sms, bps, tm, s, nullptr, trial_group);
+                                              num_sms, bps, tm, s, nullptr);
     }
 }
 

@@ -21,10 +21,8 @@
 //   300 (host)          3.5      0.59   0.59   0.59
 // (1M points: 40.5 -> 36.8 ms.)
 //
-// Between the two, a list shorter than the grid would still launch dozens of
-// trials per query at once although most succeed at their first (a flat
-// caster: 1.4 trials a query): pass 0 then runs t = 1 alone and pass 1 the
-// rest.
+// Where most queries succeed at their first trial, that is most of the work:
+// pass 0 then runs t = 1 alone and pass 1 the rest (TrialRule).
 #pragma once
 #include "sms_device.cuh"
 #include "sms_estimator.cuh"
@@ -32,34 +30,70 @@
 namespace sms {
 
 constexpr int kTrialOpen = 0x7fffffff;
-// Lists of at most this many grids' worth of trials run in a single pass.  A
-// pass of first trials costs one walk's latency (0.25 ms); what it saves is the
-// speculative trials of the queries that succeed at once.  Pane of 30,000
-// points (15,153 listed, 64 trials, 12 grids of 4 blocks per SM): one pass
-// 0.76 ms, two passes 0.74 ms (1.07 and 1.34 ms when its grid had 9 blocks);
-// slab of 20,011 points (14,529 listed, 128 trials, 32 grids of 3 blocks): two
-// passes 3.2 ms, one pass 3.6 ms.
+// When the first trials run in a pass of their own (lists shorter than the
+// grid's lanes only; longer ones run few trials past a success anyway).  A pass
+// costs the latency of its longest walk; what it saves is the speculative
+// trials of the queries that succeed at once.
+//   kSplitNever   single scatter: 60,000 pane points x 64 0.61 ms in two passes,
+//                 0.55 in one; 600,000 points of the 512^2 water x 100 17.6 and
+//                 17.0
+//   kSplitLong    chains and the two-stage solver, whose walks are long, for more
+//                 than kTrialSinglePass grids' worth of trials: 20,011 slab
+//                 points x 128 (14,529 listed, 32 grids of 3 blocks) 3.2 ms in
+//                 two passes, 3.6 in one; two-stage pane, 90,000 x 32 (19 grids)
+//                 0.90 and 0.96, 30,000 x 64 (12) 0.60 in one
+//   kSplitAlways  deterministic seeds (mnee_init): every trial of a query is the
+//                 same walk, so that the first one decides: 45,000 points of
+//                 the 128^2 water x 32 1.53 ms in one pass, 0.82 in two
+enum TrialSplit : int { kSplitNever, kSplitLong, kSplitAlways };
 constexpr unsigned kTrialSinglePass = 16;
 
+// How a launch runs its stream.
+struct TrialRule {
+    TrialSplit split = kSplitLong;
+    // Warps over which a stream of less than 32 trials a warp spreads, 0: the
+    // grid's (lanes of one warp wait for each other's rays, so the fewer the
+    // better while walks wait for tree nodes).
+    int warps = 0;
+    // Whether next() may hand out fewer trials than wanted before the pass ends.
+    bool even_end = false;
+    // Size of a claim: by what a trial of every query is to all warps, growing
+    // while a warp finds no open trial (30,000 two-stage pane points 0.75 ms,
+    // 0.60), or by the warp's share of the whole stream (chains: 20,011 slab
+    // points 3.22 ms, 3.19).
+    bool claim_by_row = false;
+};
+// Single-scatter scenes of at most this many triangles spread over
+// kSmallTreeWarps warps an SM: their walks wait for little and are bound by
+// instruction issue, where more warps only get in each other's way.  3,000
+// points x 32, over the grid's 36 warps an SM / 8 / 4 / 2: sphere 0.208 / 0.192
+// / 0.175 / 0.178 ms, water of 18 triangles 0.398 / 0.360 / 0.340 / 0.325, of
+// 450 0.422 / 0.414 / 0.403 / 0.390, of 1,922 0.486 / 0.483 / 0.484 / 0.504.
+constexpr uint32_t kSmallTree = 512;
+constexpr int kSmallTreeWarps = 2;
+// Rounds a claim grows to while a warp finds no open trial.
+constexpr unsigned kTrialClaimMax = 8;
+
 // Trials [lo, hi] of one pass, and the lanes of a warp that take part (`most`
-// at most): fewer when all of the pass's trials fit the grid that way (lanes
-// of one warp wait for each other's rays).
+// at most).
 struct TrialPlan {
     int lo, hi;
     int lanes;
 };
 
-SMS_D TrialPlan trial_plan(unsigned n_list, int cap, int pass, int most) {
+SMS_D TrialPlan trial_plan(unsigned n_list, int cap, int pass, int most, TrialRule rule) {
     const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x / 32), all = 32ull * warps;
     const unsigned long long jobs = (unsigned long long)n_list * (unsigned)cap;
-    const bool split = n_list < all && jobs > kTrialSinglePass * all;
+    const bool split = n_list < all && (rule.split == kSplitAlways ||
+                                        (rule.split == kSplitLong && jobs > kTrialSinglePass * all));
     TrialPlan p;
     p.lo = 1;
     p.hi = cap;
     if (pass == 0) p.hi = split ? 1 : 0;
     else if (split) p.lo = 2;
     const unsigned long long mine = (unsigned long long)n_list * (unsigned)max(0, p.hi - p.lo + 1);
-    p.lanes = (int)min((unsigned long long)most, max(1ull, (mine + warps - 1) / warps));
+    const unsigned long long over = rule.warps > 0 ? min(warps, (unsigned long long)rule.warps) : warps;
+    p.lanes = (int)min((unsigned long long)most, max(1ull, (mine + over - 1) / over));
     return p;
 }
 
@@ -75,35 +109,64 @@ struct TrialStream {
     unsigned long long total;
     unsigned n_list;
     TrialPlan plan;
+    TrialRule rule;
     int ready = 0;       // buffered trials
+    unsigned rounds = 1; // of the last claim
+    bool claimed = false, found = true;   // whether there was one, and an open trial in it
     bool drained = false;
 
-    SMS_D TrialStream(unsigned n, int cap, int pass, int most = 32) : n_list(n), plan(trial_plan(n, cap, pass, most)) {
+    SMS_D TrialStream(unsigned n, int cap, int pass, int most = 32, TrialRule r = TrialRule())
+        : n_list(n), plan(trial_plan(n, cap, pass, most, r)), rule(r) {
         total = (unsigned long long)n * (unsigned)max(0, plan.hi - plan.lo + 1);
     }
 
     // Draw up to `want` trials (at most 32), in stream order, for the lanes
     // of rank < want; returns whether this lane got one.  Called by the whole
-    // warp.  Fewer than want: the pass has no more.
+    // warp.  Fewer than want: the pass has no more (or rule.even_end).
     SMS_D bool next(TrialBuffer &buf, const uint32_t *list, const int *count, DevCounters *ctr, int pass,
                     int chunk, int want, int rank, uint32_t &qi, int &t) {
         const unsigned full = 0xffffffffu;
         const int lane = (int)(threadIdx.x & 31);
-        while (ready < want && !drained) {
+        const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x / 32);
+        int goal = want;
+        while (ready < goal && !drained) {
             if (cur >= end) {
-                // a claim is a few rounds of the warp (chunk at least), but no
-                // more than its share of the stream
-                const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x / 32);
-                const unsigned long long share = total / (4 * warps) / plan.lanes;
-                const unsigned claim = (unsigned)plan.lanes * (unsigned)max((unsigned long long)chunk, min(4ull, max(1ull, share)));
+                // A claim is one to four rounds of the warp, chunk at least.
+                const unsigned long long grid = warps * (unsigned)plan.lanes;
+                const unsigned share = (unsigned)min(4ull, rule.claim_by_row ? n_list / grid : total / (4ull * grid));
+                rounds = max(max(found || !rule.claim_by_row ? 1u : min(2u * rounds, kTrialClaimMax), share),
+                             (unsigned)chunk);
+                found = false;
+                unsigned claim = (unsigned)plan.lanes * rounds;
                 // Once every query has a success the warp stops, and it looks
                 // before it claims: a claimed range is never dropped, because it
                 // can hold a trial before a success that another warp found in
                 // a later range in the meantime.  All ranges before a success
-                // then belong to warps that run them.
+                // then belong to warps that run them.  The first claim does not
+                // look: all warps make it at once, and with a look before it
+                // those near the counter took the whole of a short stream
+                // (100 points of the 512^2 water 0.60 ms, without 0.53).
                 unsigned long long got = total;
-                if (lane == 0 && *(volatile unsigned *)&ctr->trial_done < n_list)
-                    got = atomicAdd(&ctr->trial_jobs[pass], (unsigned long long)claim);
+                if (lane == 0) {
+                    bool more = true;
+                    if (claimed) {
+                        more = *(volatile unsigned *)&ctr->trial_done < n_list;
+                        // The last part of a short stream goes to all warps, a
+                        // few trials each, instead of full warps that run it for
+                        // a whole walk of 32 diverging lanes (115,000 points of
+                        // the 512^2 water x 32, 1.06 grids of trials: 3.73 ms,
+                        // shared out 2.95).
+                        if (rule.even_end && total <= 64ull * warps) {
+                            const unsigned long long at = *(volatile unsigned long long *)&ctr->trial_jobs[pass];
+                            const unsigned long long left = at < total ? 4ull * (total - at) / warps : 0ull;
+                            if (left < claim) claim = (unsigned)max(1ull, left);
+                        }
+                    }
+                    if (more) got = atomicAdd(&ctr->trial_jobs[pass], (unsigned long long)claim);
+                }
+                claimed = true;
+                claim = __shfl_sync(full, claim, 0);
+                if (rule.even_end) goal = min(goal, (int)claim);
                 cur = __shfl_sync(full, got, 0);
                 end = min(cur + claim, total);
                 if (cur >= total) { drained = true; break; }
@@ -120,6 +183,7 @@ struct TrialStream {
                 open = *(volatile const int *)(count + q) > tt;
             }
             const unsigned m = __ballot_sync(full, open);
+            found = found || m != 0u;
             if (open) {
                 const int at = ready + __popc(m & ((1u << lane) - 1u));
                 buf.qi[at] = q;
@@ -211,7 +275,8 @@ inline uint32_t first_walk_blocks(uint32_t n, int lanes) { return ((n - 1) / (ui
 
 // Whether a pass of first trials may run at all for a batch of n queries on a
 // grid of `blocks` blocks (trial_plan decides by the list's length).
-inline bool trial_split_possible(uint32_t n, int cap, int blocks) {
+inline bool trial_split_possible(TrialRule rule, uint32_t n, int cap, int blocks) {
+    if (rule.split != kSplitLong) return rule.split == kSplitAlways;
     return (unsigned long long)n * (unsigned)cap > (unsigned long long)kTrialSinglePass * 128u * (unsigned)blocks;
 }
 
