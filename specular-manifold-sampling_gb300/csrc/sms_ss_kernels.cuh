@@ -32,7 +32,7 @@ namespace sms {
 // Normal-mapped casters: the map's frame and the two-stage solver add
 // arithmetic, not traversal, so what counts is that the step stays in
 // registers.  4 blocks (128 registers); pane of 30,000 points with the
-// two-stage solver at 4 / 5 / 6 / 9 blocks: 0.76 / 0.80 / 0.91 / 1.06 ms.
+// two-stage solver at 4 / 5 / 6 / 9 blocks: 0.60 / 0.75 / 0.86 / 1.05 ms.
 constexpr int ss_walk_blocks(int var) { return (var & 4) ? 4 : SMS_SS_WALK_MIN_BLOCKS; }
 
 // The same of the biased estimator's kernel for large batches (see below), and
@@ -409,7 +409,8 @@ cudaError_t ss_caster_launch(const DevScene &sc, const SolverCfg &cfg, int c, co
     const int tblocks = num_sms * (bps > 0 ? bps : ss_walk_blocks(kVar));
     const int cap = cfg.max_trials > 0 ? cfg.max_trials : kTrialHardLimit;
     TrialRule rule;
-    rule.split = cfg.mnee_init ? kSplitAlways : (kVar & 2) ? kSplitLong : kSplitNever;
+    // (the two-stage solver draws a slope for every walk: not deterministic)
+    rule.split = (kVar & 2) ? kSplitLong : cfg.mnee_init ? kSplitAlways : kSplitNever;
     rule.claim_by_row = true;
     rule.warps = sc.n_tris <= kSmallTree ? kSmallTreeWarps * num_sms : 0;
     rule.even_end = true;

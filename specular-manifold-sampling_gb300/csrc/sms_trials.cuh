@@ -19,7 +19,7 @@
 //   32,003              6.5 ms   3.6    3.3    3.2
 //   7,321 (64^2, 100)   2.2      1.25   1.1    0.84
 //   300 (host)          3.5      0.59   0.59   0.59
-// (1M points: 40.5 -> 36.8 ms.)
+// (1M points: 40.5 -> 36.1 ms.)
 //
 // Where most queries succeed at their first trial, that is most of the work:
 // pass 0 then runs t = 1 alone and pass 1 the rest (TrialRule).

@@ -46,6 +46,24 @@ def test_streams_of_one_and_two_grids(sms, workloads, gpu_lib, n, blocks):
     ctx.close()
 
 
+@pytest.mark.parametrize("res", [2, 16, 17, 18])
+@pytest.mark.parametrize("n", [1, 305, 2500])
+def test_small_trees(sms, workloads, gpu_lib, res, n):
+    """Trees around the size from which walks spread over all warps (512
+    triangles: 17 x 17 vertices): a query's result is the same alone, in a small
+    batch and in a larger one."""
+    W = workloads
+    q = W.water_queries(5000)
+    ctx = sms.Context(sms.Scene(W.water_scene(res=res)), sms.SMSConfig(max_trials=48))
+    ss = sms.SpecularManifoldSingleScatter(ctx)
+    whole = ss.specular_manifold_sampling(q, seed=8)
+    part = ss.specular_manifold_sampling(np.ascontiguousarray(q[:, 40:40 + n]), seed=8, stream_offset=40)
+    ctx.close()
+    assert (whole[1] > 0).any()
+    for x, y in zip(whole, part):
+        assert np.array_equal(x[..., 40:40 + n], y)
+
+
 def test_trial_group_does_not_slow_a_batch_down(sms, workloads, gpu_lib):
     """Every accepted trial group leaves the batch at its default speed (8 lanes
     a warp took 1.8 times as long) and its results as they are."""
