@@ -18,10 +18,6 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t *>(&v);
 }
-__device__ __forceinline__ float2 unpack_bf16(uint32_t u) {
-    __nv_bfloat162 v = *reinterpret_cast<__nv_bfloat162 *>(&u);
-    return __bfloat1622float2(v);
-}
 
 // D += A (16x16 bf16, row-major) * B (16x8 bf16, column-major), FP32 accumulate.
 __device__ __forceinline__ void mma16816(float d[4], const uint32_t a[4], uint32_t b0, uint32_t b1) {

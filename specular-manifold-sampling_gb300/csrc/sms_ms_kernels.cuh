@@ -35,12 +35,18 @@ namespace sms {
 
 constexpr unsigned kFull = 0xffffffffu;
 // Ended lanes of a warp before chain_run hands out new walks: 20,011 slab
-// points, unbiased, at 4 / 8 / 16 / 32 (a round of walks at a time) 3.42 / 3.47
-// / 3.55 / 4.05 ms.
+// points x 128, unbiased, at 4 / 8 / 16 / 32 (a round of walks at a time) 3.18 /
+// 3.30 / 3.40 / 3.97 ms.
 constexpr int kChainRefill = 4;
-// Blocks per SM of the trial kernel: what 168 registers (chains of two) let
-// reside.  More blocks with fewer registers lose to spills: 20,011 slab points
-// at 3 / 4 / 5 / 6 / 8 blocks 4.1 / 4.5 / 5.0 / 5.4 / 6.2 ms.
+// Blocks per SM of the trial kernel: what 168 registers let reside.  More blocks
+// with fewer registers lose to spills.  20,011 points, unbiased, ms a call at 2 /
+// 3 / 4 / 5 / 6 / 8 blocks (with one warp per query and no bound before):
+//   slab x 128           3.14 / 3.18 / 3.30 / 3.54 / 4.01 / 4.27   (9.2)
+//   one vertex x 64      0.81 / 0.80 / 0.84 / 0.93 / 1.04 / 1.21   (1.3)
+//   three vertices x 64  4.67 / 4.68 / 4.78 / 5.11 / 5.36 / 6.12   (13.8)
+//   four vertices x 64   7.52 / 7.94 / 8.38 / 8.11 / 8.56 / 9.45   (39.5)
+//   two rough x 64       3.15 / 3.23 / 3.43 / 3.36 / 3.58 / 4.02   (12.0)
+//   four rough x 64      8.74 / 9.29 / 9.80 / 9.48 / 10.0 / 10.9   (46.4)
 constexpr int kMsWalkBlocks = 3;
 
 SMS_D M2 mmul(M2 a, M2 b) { return {a.a * b.a + a.b * b.c, a.a * b.b + a.b * b.d, a.c * b.a + a.d * b.c, a.c * b.b + a.d * b.d}; }
@@ -384,6 +390,20 @@ SMS_D bool chain_step(const SolverCfg &cfg, f3 x0, f3 lp, const Chain<K> &c, boo
     return true;
 }
 
+// Admissibility of a converged chain: every vertex reflects or refracts as its
+// ior says (newton_solver :476-497).
+template <int K>
+SMS_D bool chain_admissible(f3 x0, f3 lp, const Chain<K> &c) {
+    #pragma unroll
+    for (int i = 0; i < K; ++i) {
+        f3 xp = i == 0 ? x0 : c.v[i - 1].p, xn = i == K - 1 ? lp : c.v[i + 1].p;
+        f3 wi = normalize(xp - c.v[i].p), wo = normalize(xn - c.v[i].p);
+        bool refraction = dot(c.v[i].gn, wi) * dot(c.v[i].gn, wo) < 0.f;
+        if ((c.v[i].eta == 1.f) ? refraction : !refraction) return false;
+    }
+    return true;
+}
+
 // newton_solver (:410-498).  c holds the seed path on entry and the solution
 // on success; tmpl = the estimate's template shapes.
 template <int K, bool kNM = false, bool kRough = false, ChainForm kForm = kChainLoop>
@@ -426,29 +446,7 @@ SMS_D bool chain_newton(const DevScene &sc, const SolverCfg &cfg, f3 x0, f3 lp, 
         beta = need ? fminf(1.f, 2.f * beta) : 0.5f * beta;
         it++;
     }
-    if (!(ok && conv)) return false;
-    #pragma unroll
-    for (int i = 0; i < K; ++i) {
-        f3 xp = i == 0 ? x0 : c.v[i - 1].p, xn = i == K - 1 ? lp : c.v[i + 1].p;
-        f3 wi = normalize(xp - c.v[i].p), wo = normalize(xn - c.v[i].p);
-        bool refraction = dot(c.v[i].gn, wi) * dot(c.v[i].gn, wo) < 0.f;
-        if ((c.v[i].eta == 1.f) ? refraction : !refraction) return false;
-    }
-    return true;
-}
-
-// Admissibility of a converged chain: every vertex reflects or refracts as its
-// ior says (newton_solver :476-497).
-template <int K>
-SMS_D bool chain_admissible(f3 x0, f3 lp, const Chain<K> &c) {
-    #pragma unroll
-    for (int i = 0; i < K; ++i) {
-        f3 xp = i == 0 ? x0 : c.v[i - 1].p, xn = i == K - 1 ? lp : c.v[i + 1].p;
-        f3 wi = normalize(xp - c.v[i].p), wo = normalize(xn - c.v[i].p);
-        bool refraction = dot(c.v[i].gn, wi) * dot(c.v[i].gn, wo) < 0.f;
-        if ((c.v[i].eta == 1.f) ? refraction : !refraction) return false;
-    }
-    return true;
+    return ok && conv && chain_admissible<K>(x0, lp, c);
 }
 
 // dp_du du + dp_dv dv, the second product fused (chains of one vertex; see ChainForm).
@@ -526,7 +524,7 @@ SMS_D void chain_run(const DevScene &sc, const SolverCfg &cfg, int lanes, uint32
                 go = !w.seed;
                 w.beta = 0.5f * w.beta;
             }
-            // the last iteration's chain, from which no step would be taken, is counted, not traced
+            // the last iteration, from whose chain no step would be taken, is counted; its chain is not traced
             if (go && ++w.it >= cfg.max_iterations) go = false;
             if (go) {
                 w.target = w.vp - w.step * (cfg.step_scale * w.beta);
