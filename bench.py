@@ -724,7 +724,10 @@ def run_ours(args):
                                "treelet_nodes": tuned["best"][2], "queue_chunk": tuned["best"][3],
                                "autotune_ms": tuned["ms"]} if tuned else "library default")},
         "walks_per_s": world * st["walks"] / total_s,
+        # iterations of speculative trials that ended before their query's success included
         "newton_iterations_per_walk": st["newton_iterations"] / max(1, st["walks"]),
+        "newton_iterations_note": "per counted walk; speculative trials that ended before their query's success "
+                                  "are in the iterations, not in the walks",
         "trials_per_connection": st["bernoulli_trial_iterations"] / max(1, st["bernoulli_trial_calls"]),
         "converged_fraction_first_walk": st["solver_succeeded"] / max(1, st["solver_succeeded"] + st["solver_failed"]),
         "rays_per_s": world * st["rays"] / total_s,

@@ -347,9 +347,10 @@ static_assert(smb_off(kLayers - 1) == smb_off(1) + (kLayers - 2) * kHidden * (kH
               "hidden layers are evenly spaced");
 
 // Samples a warp of mlp_wgrad_kernel sums up (the last one of a tile fewer).
-// 8,192 samples at 128 / 256 / 512 / 1024: 113 / 110 / 111 / 112 us a gradient:
-// longer chunks leave warps idle, shorter ones add more atomics.  A chunk that
-// had to divide the batch was 32 samples at 31,712 (529 us, now 235).
+// 8,192 samples at 128 / 256 / 512 / 1024: 88.6 / 86.5 / 88.6 / 89.9 us a
+// gradient, 31,712 samples 201 / 183 / 175 / 173: longer chunks leave warps idle
+// in small batches, shorter ones add more atomics.  A chunk that had to divide
+// the batch was 32 samples at 31,712 (529 us).
 constexpr int kWgradChunk = 256;
 
 // dW_l[o][i] += sum_b dz_l[b][o] h_l[b][i] over one batch chunk; one warp per

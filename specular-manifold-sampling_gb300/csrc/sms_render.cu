@@ -30,7 +30,7 @@
 // One host read per bounce (query and live-path counts) drives the loop.
 // Every sum runs in a fixed order, so images are bit-reproducible, and since
 // all random numbers are keyed by path and bounce they do not depend on the
-// wavefront size.
+// wavefront size, but for the order of a pixel's sum over its samples.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
